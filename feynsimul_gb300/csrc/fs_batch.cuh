@@ -123,9 +123,9 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
         FsbStream g, ws;
         {
 #if FSB_RANLUX
-            fs_rl_load(g.st, sd.rtab + (size_t)th * 28);
+            fs_rl_load<FS_NSKIP>(g.st, sd.rtab + (size_t)th * 28);
             g.count = 0u;
-            fs_rl_load(ws.st, sd.gtab + (size_t)w * 28);
+            fs_rl_load<FS_NSKIP>(ws.st, sd.gtab + (size_t)w * 28);
             ws.count = 0u;
 #else
             const uint4 s4 = *(const uint4 *)(sd.seeds + (size_t)th * 4);
@@ -246,8 +246,8 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
         }
         sd.accepts[th] = n_acc;
 #if FSB_RANLUX
-        fs_rl_store(g.st, sd.rtab + (size_t)th * 28);
-        if (t == 0) fs_rl_store(ws.st, sd.gtab + (size_t)w * 28);
+        fs_rl_store<FS_NSKIP>(g.st, sd.rtab + (size_t)th * 28);
+        if (t == 0) fs_rl_store<FS_NSKIP>(ws.st, sd.gtab + (size_t)w * 28);
 #else
         *(uint4 *)(sd.seeds + (size_t)th * 4) = make_uint4(g.x, g.y, g.z, g.w);
         if (t == 0) *(uint4 *)(sd.wseeds + (size_t)w * 4) = make_uint4(ws.x, ws.y, ws.z, ws.w);

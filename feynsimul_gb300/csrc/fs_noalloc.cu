@@ -36,7 +36,7 @@ __global__ void fs_ranlux_init_scratch_kernel(fs_u32 *tab, const fs_u64 *xs, int
     if (i >= n) return;
     FsRanlux r;
     fs_rl_seed(r, xs[i]);
-    fs_rl_store(r, tab + (size_t)i * 28);
+    fs_rl_store_new<0>(r, tab + (size_t)i * 28);
 }
 
 extern int fsi_thread_error(int code, const char *msg);

@@ -738,7 +738,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
         FsUStream fs;
 #if FS_RANLUX
         if (mover) {
-            fs_rl_load(fs.st, a.rtab + (size_t)tid * 28);
+            fs_rl_load<FS_NSKIP>(fs.st, a.rtab + (size_t)tid * 28);
             fs.count = 0u;
         }
         // The walker's offset stream: every reference work-item of the walker advances an
@@ -746,9 +746,9 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
         FsIStream &is = s_istream[wl];
         if (mover && t == 0) {
 #if FS_COMPAT
-            fs_rl_load(is.st, a.gtab + (size_t)tid * 28);
+            fs_rl_load<FS_NSKIP>(is.st, a.gtab + (size_t)tid * 28);
 #else
-            fs_rl_load(is.st, a.gtab + (size_t)w * 28);
+            fs_rl_load<FS_NSKIP>(is.st, a.gtab + (size_t)w * 28);
 #endif
             is.count = 0u;
 #if FS_OFF_PRE
@@ -1335,12 +1335,12 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
         }
 #endif
 #if FS_RANLUX
-        if (mover) fs_rl_store(fs.st, a.rtab + (size_t)tid * 28);
+        if (mover) fs_rl_store<FS_NSKIP>(fs.st, a.rtab + (size_t)tid * 28);
         FS_WSYNC();
 #if FS_COMPAT
-        if (mover) fs_rl_store(is.st, a.gtab + (size_t)tid * 28);
+        if (mover) fs_rl_store<FS_NSKIP>(is.st, a.gtab + (size_t)tid * 28);
 #else
-        if (mover && t == 0) fs_rl_store(is.st, a.gtab + (size_t)w * 28);
+        if (mover && t == 0) fs_rl_store<FS_NSKIP>(is.st, a.gtab + (size_t)w * 28);
 #endif
 #else
         if (mover) *(uint4 *)(a.seeds + (size_t)tid * 4) = make_uint4(fs.x, fs.y, fs.z, fs.w);
@@ -1392,7 +1392,7 @@ extern "C" __global__ void fs_ranlux_init(fs_u32 *tab, const fs_u64 *xs, int n)
     if (i >= n) return;
     FsRanlux r;
     fs_rl_seed(r, xs[i]);
-    fs_rl_store(r, tab + (size_t)i * 28);
+    fs_rl_store_new<0>(r, tab + (size_t)i * 28);
 }
 
 // stream dumps used by the RNG parity tests
@@ -1409,7 +1409,7 @@ extern "C" __global__ void fs_ranlux_dump(const fs_u64 *xs, int n, int n_calls, 
         float *o = out + ((size_t)i * n_calls + c) * 4;
         o[0] = o0; o[1] = o1; o[2] = o2; o[3] = o3;
     }
-    fs_rl_store(r, states + (size_t)i * 28);
+    fs_rl_store_new<FS_NSKIP>(r, states + (size_t)i * 28);
 }
 
 extern "C" __global__ void fs_ranlux_dump64(const fs_u64 *xs, int n, int n_calls, double *out)
