@@ -213,17 +213,44 @@ __device__ __forceinline__ fs_u32 fs_offset(FsIStream &g, fs_u32 range)
 #define FS_OLD_N 1
 #endif
 
-// Rolled move loops for RANLUX (its generator calls are large) and for big plugins (a
-// fully unrolled move repeats the potential 2 * (2^S - 1) times, which for a 10-atom
-// cluster costs minutes of compilation and overflows the instruction cache)
+// How far the move's loops are unrolled: FS_NODE_UNROLL the nodes of a level, FS_DOF_UNROLL a
+// node's degrees of freedom, FS_ACT_UNROLL the old- and new-action loops (2^S - 1 potential
+// evaluations each).  A move unrolled in full overlaps the nodes' latencies, until its code
+// leaves the instruction cache.  FS_MOVE_CODE estimates its instructions: about 30 a degree
+// and node for Box-Muller in fast math and 180 in IEEE (log, sin and sqrt inline), 10 a node
+// for a potential of one or two degrees, 50 a degree for larger ones (LM2M2 trimer).
+// Measured, unrolled / rolled, us a run: oscillator S = 6 fast (2520) 509 / 579 and S = 7 (5080)
+// 1142 / 1105, IEEE S = 4 (2850) 428 / 513, S = 5 (5890) 665 / 648, S = 6 (11970) 2540 / 1053;
+// trimer xorshift fast S = 2 (1440) 470 / 492, S = 3 (3360) 679 / 647, S = 4 (7200) 1038 / 755;
+// trimer IEEE S = 2 (4140) 735 / 614, S = 3 (9660) 3127 / 1413, S = 4 (20700) 6655 / 2969: the
+// line lies at 3000.  Rolled, a fast trimer gains 1 % from two nodes at a time, an IEEE one loses
+// 9 % (its six degrees fill the cache), and a cheap potential wants its action loop unrolled
+// (oscillator IEEE S = 6: 1053 against 1326).
+// RANLUX (its generator calls are large) and more than 8 degrees of freedom are always rolled.
+#define FS_MOVE_CODE ((FS_SEG - 1) * (FS_DOF * (FS_FAST ? 30 : 180) + (FS_DOF < 3 ? 10 : 50 * FS_DOF)))
 #if FS_RANLUX || FS_DOF > 8
 #define FS_MOVE_UNROLL _Pragma("unroll 1")
-#else
+#define FS_NODE_UNROLL _Pragma("unroll 1")
+#define FS_DOF_UNROLL _Pragma("unroll 1")
+#define FS_ACT_UNROLL _Pragma("unroll 1")
+#elif FS_MOVE_CODE <= 3000
 #define FS_MOVE_UNROLL _Pragma("unroll")
+#define FS_NODE_UNROLL _Pragma("unroll")
+#define FS_DOF_UNROLL _Pragma("unroll")
+#define FS_ACT_UNROLL _Pragma("unroll")
+#else
+#define FS_MOVE_UNROLL _Pragma("unroll 1")
+#define FS_DOF_UNROLL _Pragma("unroll")
+#if FS_DOF < 3
+#define FS_NODE_UNROLL _Pragma("unroll 2")
+#define FS_ACT_UNROLL _Pragma("unroll 16")
+#elif FS_FAST
+#define FS_NODE_UNROLL _Pragma("unroll 2")
+#define FS_ACT_UNROLL _Pragma("unroll 2")
+#else
+#define FS_NODE_UNROLL _Pragma("unroll 1")
+#define FS_ACT_UNROLL _Pragma("unroll 1")
 #endif
-// The old- and new-action loops (2^S - 1 potential evaluations each)
-#ifndef FS_ACT_UNROLL
-#define FS_ACT_UNROLL FS_MOVE_UNROLL
 #endif
 
 // kernel.c:258-399 on a shared-memory path P[DOF][N].
@@ -284,7 +311,7 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
     for (int n = 1; n <= FS_S; n++) {
         const int half = 1 << (FS_S - n);
         const FT sig = sigma[n];
-        FS_MOVE_UNROLL
+        FS_NODE_UNROLL
         for (int i = 0; i < (1 << (n - 1)); i++) {
             const fs_u32 m = ((fs_u32)((1 + 2 * i) * half) + start) & (FS_N - 1);
             const fs_u32 l = ((fs_u32)(i * 2 * half) + start) & (FS_N - 1);
@@ -298,7 +325,7 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
                 const FT u = uv[2 * d];
                 const FT v = uv[2 * d + 1];
 #else
-            FS_MOVE_UNROLL
+            FS_DOF_UNROLL
             for (int d = 0; d < FS_DOF; d++) {
                 const FT u = fs_uniform(g);
                 const FT v = fs_uniform(g);
