@@ -360,12 +360,13 @@ static std::string gen_source(const fs_handle &h, const std::string &potential,
     o << "\n// ---- random number generators ----\n" << kRngSrc << "\n";
     if (c.learned) o << "\n// ---- learned proposal network ----\n" << kMlpSrc << "\n";
     o << "\n// ---- plugin userCode ----\n" << cvt(user_code) << "\n";
-    std::ostringstream args, at;
+    std::ostringstream args, at, of;
     for (int i = 0; i < c.dof; i++) {
         args << (i ? ", " : "") << "FT x" << (i + 1);
         at << (i ? ", " : "") << "FS_AT(P, " << i << ", (i))";
+        of << (i ? ", " : "") << "(x)[" << i << "]";
     }
-    o << "#define FS_ARGS_AT(P, i) " << at.str() << "\n";
+    o << "#define FS_ARGS_AT(P, i) " << at.str() << "\n#define FS_ARGS_OF(x) " << of.str() << "\n";
     // Plugins of more than 8 DOF (clusters of 4+ atoms, tens of pair terms) are called, not
     // inlined: the sweep evaluates the potential at several places, and inlined copies of a
     // 45-pair potential overflow the instruction cache (measured: +19% to +47% on a 10-atom
@@ -532,6 +533,58 @@ static int device_sms()
     return sms;
 }
 
+static long long round16(long long words) { return (words + 15) / 16 * 16; }
+
+// Shared memory of one sweep CTA: the walkers' paths and potential cache (each region a whole
+// number of 16 words), the correlator buffers and the histogram.
+static size_t sweep_smem(const fs_handle &h, long long vstride, size_t hist_bytes)
+{
+    const long long path = h.cfg.global_path ? 0 : round16(h.wpb * h.wstride);
+    return (size_t)(path + round16(h.wpb * vstride) + h.wpb * h.cwstride) * h.ft + hist_bytes;
+}
+
+// Walkers per CTA of a sweep without correlator helpers: CTAs of 128 threads, at most 100 KB of
+// shared memory, and where the walkers are so few that some SMs would get no CTA, fewer per CTA
+// down to a warp of threads (444 bound trimers, 8 threads each: 747 us a run in 28 CTAs of 4
+// warps, 719 in 111 of one).  One-thread walkers take CTAs of one warp (60000 oscillators: 1178
+// us with two warps, 1103 with one), and fewer lanes than a warp where that fills more SMs: the
+// lanes of a warp wait for one another's branches (a path shift's length, a rejection).  With
+// potentials of one or two degrees that pays down to one lane, until every scheduler has a CTA
+// (2048 oscillators 374 us at 32 lanes, 300 at 8, 280 at 2; 100 oscillators 370 at 32, 267 at 4,
+// 200 at one); clusters stop at four lanes and a CTA per SM, since their code does not stay in
+// the instruction cache (5 atoms: 634 at 4, 824 at one).
+static int default_wpb(const fs_handle &h, size_t per_walker, size_t hist_bytes)
+{
+    if (h.tpw > 32) return 1;
+    int wpb = std::max(1, (h.tpw == 1 ? 32 : 128) / h.tpw);
+    while (wpb > 1 && per_walker * wpb + hist_bytes > 100 * 1024) wpb /= 2;
+    const bool single = h.tpw == 1, cheap = h.cfg.dof <= 2;
+    const int least = !single ? 32 : cheap ? 1 : 4, ctas = single && cheap ? 4 * device_sms() : device_sms();
+    while (wpb * h.tpw > least && (h.cfg.n_walkers + wpb - 1) / wpb < ctas) wpb /= 2;
+    return wpb;
+}
+
+// The reference's enableGlobalPath says where its kernel keeps the paths; the results are the
+// same bit for bit.  Shared memory is the faster place wherever it holds every walker of the
+// launch at once or 384 threads per SM (us a run, device memory / shared memory: trimer N = 128,
+// 444 walkers 160 / 122; N = 1024, 4096 walkers 2660 / 978; 10 atoms N = 256, 384 threads per SM
+// 1604 / 1297; oscillator walker moves N = 1024 2238 / 700).  With 128 to 256 threads per SM it
+// is a loss (10 atoms, N = 512, FP64: 12082 / 12718), and with correlators, whose lag sums want
+// more warps than that (10 atoms, N = 256: 1144 / 1248), the path stays where it was asked for;
+// also where the caller's register budget counts on more CTAs than shared memory admits.
+static bool path_in_shared(const fs_handle &h, size_t path_bytes, size_t hist_bytes)
+{
+    const fs_config &c = h.cfg;
+    if (!h.cors.empty()) return false;
+    const int wpb = std::min(c.walkers_per_block > 0 ? c.walkers_per_block : default_wpb(h, path_bytes, hist_bytes),
+                             c.n_walkers);
+    const size_t smem = path_bytes * wpb + 2 * 16 * h.ft + hist_bytes;
+    if (smem > 227 * 1024) return false;
+    const long long ctas = std::min((227ll * 1024) / (long long)(smem + 1024), 2048ll / (wpb * h.tpw));
+    if (ctas < std::max(1, c.min_blocks_per_sm)) return false;
+    return ctas * device_sms() * wpb >= c.n_walkers || ctas * wpb * h.tpw >= 384;
+}
+
 static int validate(const fs_config &c, int nops, int ncor, int nhist)
 {
     if (c.dof < 1 || c.dof > 256) return fail(nullptr, FS_ERR_CONFIG, "DOF must be in [1, 256]");
@@ -691,17 +744,25 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         h->cwstride = cw;
     }
     // padded shared-memory path (see FS_PHYS in fs_pimc.cuh): one word after every 2^S
-    // slices; the walker stride is an odd multiple of 16 words
+    // slices, so a walker's segment threads, t, read words o = 2^S + 1 apart; the stride of
+    // the 32 / T walkers that share a warp is T o modulo 32, which gives the 32 lanes the 32
+    // multiples of o and so distinct banks (one-thread walkers with a stride of 16 words met in
+    // two banks: 60000 oscillators in walker mode took 1486 us a run, 1178 with this).
     const long long dstride = c.n_slices + (c.n_slices >> c.bisection_level);
-    long long wstride = (long long)c.dof * dstride;
-    wstride = ((wstride + 15) / 16) * 16;
-    if ((wstride / 16) % 2 == 0) wstride += 16;
+    auto spread = [&](long long words) {
+        if (h->tpw >= 32) return round16(words);
+        const long long want = (h->tpw * ((1ll << c.bisection_level) + 1)) % 32;
+        return words + (want - words % 32 + 32) % 32;
+    };
+    long long wstride = spread((long long)c.dof * dstride);
+    const size_t hist_bytes = (size_t)(c.hist_bins > 0 && !h->hists.empty() ? c.hist_bins : 0) * 4;
+    // potential cache: one value per slice in the path's padded slice layout
+    const long long vstride = spread(dstride);
+    if (c.global_path &&
+        path_in_shared(*h, (size_t)(wstride + (c.potential_cache == 1 ? vstride : 0)) * h->ft, hist_bytes))
+        h->cfg.global_path = 0;
     if (c.global_path) wstride = (long long)c.dof * c.n_slices;  // no shared-memory path
     h->wstride = wstride;
-    // potential cache: one value per slice in the path's padded slice layout, walker stride
-    // an odd multiple of 16 words
-    long long vstride = ((dstride + 15) / 16) * 16;
-    if ((vstride / 16) % 2 == 0) vstride += 16;
     const size_t per_walker_base =
         (size_t)((c.global_path ? 0 : wstride) + h->cwstride) * h->ft;
     // the path-shift and single-node moves change slices outside the bisection's
@@ -709,8 +770,7 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
     const bool other_moves = (c.moves & (FS_MOVE_PATH_SHIFT | FS_MOVE_SINGLE_NODE)) != 0;
     h->vstride = (c.potential_cache == 2 || c.potential_cache == 3 || other_moves) ? 0 : vstride;
     h->vglobal = c.potential_cache == 3 && !other_moves ? 1 : 0;
-    size_t per_walker = per_walker_base + (size_t)h->vstride * h->ft;
-    const size_t hist_bytes = (size_t)(c.hist_bins > 0 && !h->hists.empty() ? c.hist_bins : 0) * 4;
+    const size_t per_walker = per_walker_base + (size_t)h->vstride * h->ft;
     if (c.walkers_per_block > 0) {
         h->wpb = c.walkers_per_block;
     } else if (h->mx > 1) {
@@ -722,12 +782,8 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         h->wpb = h->pipe ? step : std::max(1, 128 / (h->tpw * h->mx));
         while (h->wpb > step && (c.n_walkers % h->wpb || per_walker * h->wpb + hist_bytes > 100 * 1024))
             h->wpb -= step;
-    } else if (h->tpw > 32) {
-        h->wpb = 1;
     } else {
-        int target = h->tpw == 1 ? 64 : 128;
-        h->wpb = std::max(1, target / h->tpw);
-        while (h->wpb > 1 && per_walker * h->wpb + hist_bytes > 100 * 1024) h->wpb /= 2;
+        h->wpb = default_wpb(*h, per_walker, hist_bytes);
     }
     h->wpb = std::min(h->wpb, c.n_walkers);
     if (h->tpw > 32 && h->wpb != 1) {
@@ -754,25 +810,30 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         return fail(nullptr, FS_ERR_CONFIG, "walkers_per_block * threads per walker exceeds 1024");
     }
     h->grid = (c.n_walkers + h->wpb - 1) / h->wpb;
-    h->smem = per_walker * h->wpb + hist_bytes;
+    h->smem = sweep_smem(*h, h->vstride, hist_bytes);
     if (h->vstride && c.potential_cache == 0) {
         // automatic: the cache halves the potential evaluations but takes shared memory;
         // keep it where it costs no resident CTA per SM, or where the potential is large
         // (more than 8 DOF: a cluster of 4+ atoms)
         auto ctas = [](size_t smem) { return (227ll * 1024) / (long long)(smem + 1024); };
-        const size_t without = per_walker_base * h->wpb + hist_bytes;
+        const size_t without = sweep_smem(*h, 0, hist_bytes);
         if (ctas(h->smem) < std::min(ctas(without), 2048ll / h->block) && c.dof <= 8) h->vstride = 0;
     }
     if (h->smem > 227 * 1024 && h->vstride && c.potential_cache != 1) h->vstride = 0;  // no room
     if (!h->vstride) {
-        per_walker = per_walker_base;
-        h->smem = per_walker * h->wpb + hist_bytes;
+        h->smem = sweep_smem(*h, 0, hist_bytes);
         // automatic: where shared memory has no room for the cache, keep it in device memory
         // (L1/L2), for potentials of 3 or more DOF and launches of more than one move; the
         // launch starts with one potential evaluation per slice
         if (c.potential_cache == 0 && !other_moves && c.dof >= 3 &&
             (long long)c.operator_runs * c.metro_steps_per_operator_run >= 2)
             h->vglobal = 1;
+    }
+    if (h->smem > 227 * 1024) {
+        // the bank spread is not worth a CTA that fits without it
+        if (!c.global_path) h->wstride = round16((long long)c.dof * dstride);
+        if (h->vstride) h->vstride = round16(dstride);
+        h->smem = sweep_smem(*h, h->vstride, hist_bytes);
     }
     // Register budget: unless the caller fixes it, compile for as many CTAs per SM as shared
     // memory admits (<= 2048 threads per SM, >= 64 registers per thread) and as the grid can
@@ -1626,7 +1687,7 @@ static int rng_module(int lux, cudaLibrary_t *lib)
          "#define FS_NOPS 0\n#define FS_NCOR 0\n#define FS_OPRUNS 1\n#define FS_MSTEPS 1\n"
          "#define FS_EPS 1.0f\n#define FS_OPNORM 1.0f\n#define FS_BINS 0\n#define FS_NHIST 0\n"
          "#define FS_HBINS 0\n#define FS_RIM 4.294967296E+09f\n#define FS_DOF 1\n"
-      << kRngSrc << "\n#define FS_ARGS_AT(P, i) (P)[(i)]\n__constant__ FT fs_sigma[1] = {0.0f};\n"
+      << kRngSrc << "\n#define FS_ARGS_AT(P, i) (P)[(i)]\n#define FS_ARGS_OF(x) (x)[0]\n__constant__ FT fs_sigma[1] = {0.0f};\n"
       << "__device__ FT fs_pot(FT x1) { return x1; }\n" << kPimcSrc;
     fs_handle tmp;
     std::string cubin, log;

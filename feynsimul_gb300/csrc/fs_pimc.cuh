@@ -104,8 +104,8 @@
 // Shared-memory path layout.  Slice s of degree d of a walker sits at d * FS_DSTRIDE +
 // FS_PHYS(s) with one padding word after every 2^S slices: the segment threads of a walker
 // read slices 2^S apart, which the padding turns into 2^S + 1 words apart, an odd stride,
-// so the threads of a warp hit distinct banks.  FS_WSTRIDE (walker stride, from the host)
-// is an odd multiple of 16 words so two walkers sharing a warp use opposite bank halves.
+// so the threads of a warp hit distinct banks.  FS_WSTRIDE (walker stride, from the host) goes
+// on in the same steps, modulo 32, from one walker of a warp to the next.
 //
 // Global-path mode (FS_GLOBAL, the reference's ENABLE_GLOBAL_PATH, kernel.c:62-70 and
 // :582-588): the walker's threads work in place on its [DOF][N] rows of the paths array
@@ -681,9 +681,9 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
     FT *s_v = (FT *)fs_smem;                                     // [WPB][VSTRIDE] (FS_VCACHE)
 #else
     FT *s_path = (FT *)fs_smem;                                  // [WPB][DOF*N]
-    FT *s_v = s_path + FS_WPB * FS_WSTRIDE;                      // [WPB][VSTRIDE] (FS_VCACHE)
+    FT *s_v = s_path + (FS_WPB * FS_WSTRIDE + 15) / 16 * 16;     // [WPB][VSTRIDE] (FS_VCACHE)
 #endif
-    FT *s_cor = s_v + FS_WPB * FS_VSTRIDE;                     // [WPB][CWSTRIDE >= NCOR * CSTRIDE]
+    FT *s_cor = s_v + (FS_WPB * FS_VSTRIDE + 15) / 16 * 16;    // [WPB][CWSTRIDE >= NCOR * CSTRIDE]
     fs_u32 *s_hist = (fs_u32 *)(s_cor + FS_WPB * FS_CWSTRIDE);  // [HBINS]
 
     const int tid_b = threadIdx.x;
