@@ -93,6 +93,16 @@
 #if FS_PIPE && !(FS_COR_FMA && FS_COR_ILV)
 #error "pipelined correlator helpers sum FP32 partials over doubled slice values"
 #endif
+// Slices whose coordinates a measurement loads at once: with one or two degrees of freedom a
+// slice's operator is a few instructions, and slice by slice the loop waits for each load
+// (1024 oscillators, x^2 after every sweep, 8 slices a thread: 118 -> 101 us a run of 100)
+#if FS_DOF > 2
+#define FS_MEAS_BATCH 1
+#elif FS_PARALLEL
+#define FS_MEAS_BATCH (FS_SEG < 8 ? FS_SEG : 8)
+#else
+#define FS_MEAS_BATCH (FS_N < 8 ? FS_N : 8)
+#endif
 #define FS_CSTRIDE (FS_COR_ILV ? 2 * FS_N : FS_N)
 #ifndef FS_CWSTRIDE
 #define FS_CWSTRIDE (FS_NCOR * FS_CSTRIDE)  // per-walker correlator buffer (the host pads it)
@@ -416,37 +426,61 @@ __device__ __forceinline__ FT fs_kin(FT a, FT b)
 #endif
 
 #if FS_PATH_SHIFT
+// Slices of a path shift that are loaded ahead of their potentials: the slices are distinct, so
+// a batch's loads need not wait for the stores of the slices before them, which the compiler
+// cannot know.  With the old values saved for the shifted slices only, in coalesced columns
+// (before: the whole row, one 32-byte sector a lane and value), 2048 oscillators of 16 slices
+// went from 485 to 300 us a run.  Larger potentials hide a load by themselves, and two copies of
+// them cost more instruction fetch than that (trimer: 232 us at one, 247 at two).
+#if FS_DOF <= 2
+#define FS_SHIFT_BATCH 4
+#else
+#define FS_SHIFT_BATCH 1
+#endif
+
 // kernel.c:407-473: shift slices left..right (cyclically) of one degree of freedom by
 // offset; returns the change of the kinetic + potential sum.  left == right shifts nothing.
-__device__ __forceinline__ FT fs_shift(FT *P, int degree, FT offset, fs_u32 left, fs_u32 right)
+// saved (fixed mode): the shifted slices' old values, value j at j * FS_NWALKERS, so the walkers
+// of a warp write consecutive words.
+__device__ __forceinline__ FT fs_shift(FT *P, int degree, FT offset, fs_u32 left, fs_u32 count, FT *saved)
 {
-    if (left == right) return (FT)0;
+    const fs_u32 right = (left + count - 1) & (FS_N - 1);
     FT kinDiff = (FT)0, potDiff = (FT)0;
-    fs_u32 ll, rr;
-    if (left < right) {
-        ll = left == 0 ? FS_N - 1 : left - 1;
-        rr = right == FS_N - 1 ? 0 : right + 1;
-    } else {
-        ll = left - 1;
-        rr = right + 1;
-    }
+    const fs_u32 ll = (left - 1) & (FS_N - 1), rr = (right + 1) & (FS_N - 1);
     kinDiff = FS_SUB(kinDiff, fs_kin(FS_AT(P, degree, left), FS_AT(P, degree, ll)));
     kinDiff = FS_SUB(kinDiff, fs_kin(FS_AT(P, degree, right), FS_AT(P, degree, rr)));
     // slices left, left+1, ... right (mod N), in the reference's order
-    const fs_u32 count = left < right ? right - left + 1 : FS_N - left + right + 1;
 #pragma unroll 1
-    for (fs_u32 j = 0; j < count; j++) {
-        const fs_u32 i = (left + j) & (FS_N - 1);
-        potDiff = FS_SUB(potDiff, fs_pot(FS_ARGS_AT(P, i)));
-        FS_AT(P, degree, i) = FS_ADD(FS_AT(P, degree, i), offset);
-        potDiff = FS_ADD(potDiff, fs_pot(FS_ARGS_AT(P, i)));
+    for (fs_u32 j0 = 0; j0 < count; j0 += FS_SHIFT_BATCH) {
+        FT x[FS_SHIFT_BATCH][FS_DOF];
+#pragma unroll
+        for (int b = 0; b < FS_SHIFT_BATCH; b++)
+#pragma unroll
+            for (int d = 0; d < FS_DOF; d++) x[b][d] = FS_AT(P, d, (left + j0 + b) & (FS_N - 1));
+#pragma unroll
+        for (int b = 0; b < FS_SHIFT_BATCH; b++) {
+            const fs_u32 j = j0 + b;
+            if (FS_SHIFT_BATCH > 1 && j >= count) break;
+            potDiff = FS_SUB(potDiff, fs_pot(FS_ARGS_OF(x[b])));
+#pragma unroll
+            for (int d = 0; d < FS_DOF; d++)
+                if (d == degree) {
+#if !FS_COMPAT
+                    saved[(size_t)j * FS_NWALKERS] = x[b][d];
+#endif
+                    x[b][d] = FS_ADD(x[b][d], offset);
+                    FS_AT(P, d, (left + j) & (FS_N - 1)) = x[b][d];
+                }
+            potDiff = FS_ADD(potDiff, fs_pot(FS_ARGS_OF(x[b])));
+        }
     }
     kinDiff = FS_ADD(kinDiff, fs_kin(FS_AT(P, degree, left), FS_AT(P, degree, ll)));
     kinDiff = FS_ADD(kinDiff, fs_kin(FS_AT(P, degree, right), FS_AT(P, degree, rr)));
     return FS_ADD(kinDiff, potDiff);
 }
 
-// kernel.c:640-666: one path-shift move of degree k % DOF; saved holds N values of scratch
+// kernel.c:640-666: one path-shift move of degree k % DOF; saved: the walker's column of
+// shift_old (see fs_shift)
 __device__ __forceinline__ int fs_path_shift_move(FT *P, unsigned long long k, FsIStream &is, FsUStream &g,
                                                   FT *saved)
 {
@@ -454,28 +488,22 @@ __device__ __forceinline__ int fs_path_shift_move(FT *P, unsigned long long k, F
     const fs_u32 left = fs_offset(is, FS_N);
     const fs_u32 right = fs_offset(is, FS_N);
     const FT offset = FS_MUL((FT)FS_PSALPHA, FS_SUB(FS_MUL((FT)2, fs_uniform(g)), (FT)1));
-#if !FS_COMPAT
-#pragma unroll 1
-    for (int i = 0; i < FS_N; i++) saved[i] = FS_AT(P, degree, i);
-#else
-    (void)saved;
-#endif
-    const FT diff = fs_shift(P, degree, offset, left, right);
+    // shifted slices; left == right shifts nothing
+    const fs_u32 count = left == right ? 0u : ((right - left) & (FS_N - 1)) + 1u;
+    const FT diff = count ? fs_shift(P, degree, offset, left, count, saved) : (FT)0;
     if (FS_EXP(FS_MUL((FT)(-FS_EPS), diff)) < fs_uniform(g)) {
 #if FS_COMPAT
         // the reference reverts by shifting again by -offset (kernel.c:654-656), which
         // leaves the rounding of x + offset - offset in the path
-        if (left != right) {
-            const fs_u32 count = left < right ? right - left + 1 : FS_N - left + right + 1;
 #pragma unroll 1
-            for (fs_u32 j = 0; j < count; j++) {
-                const fs_u32 i = (left + j) & (FS_N - 1);
-                FS_AT(P, degree, i) = FS_ADD(FS_AT(P, degree, i), -offset);
-            }
+        for (fs_u32 j = 0; j < count; j++) {
+            const fs_u32 i = (left + j) & (FS_N - 1);
+            FS_AT(P, degree, i) = FS_ADD(FS_AT(P, degree, i), -offset);
         }
 #else
-#pragma unroll 1
-        for (int i = 0; i < FS_N; i++) FS_AT(P, degree, i) = saved[i];
+#pragma unroll 4
+        for (fs_u32 j = 0; j < count; j++)
+            FS_AT(P, degree, (left + j) & (FS_N - 1)) = saved[(size_t)j * FS_NWALKERS];
 #endif
         return 0;
     }
@@ -521,7 +549,7 @@ struct FsArgs {
     fs_u64 *hist;              // [hist bins]
     int *status;               // [0] flags (FS_STATUS_*), [1] 1 + a walker that raised one
     double opnorm;
-    FT *shift_old;             // path shift, fixed mode: the shifted row before the move [walkers][N]
+    FT *shift_old;             // path shift, fixed mode: the shifted slices before the move [N][walkers]
     unsigned long long step_base;  // fixed mode: Metropolis steps of earlier launches
     const uint2 *mlp_frag;     // learned proposal: network fragments and biases
     const float *mlp_bias;
@@ -848,10 +876,10 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #endif
 
 #if FS_NOPS > 0
-        // the operators of slice s of path Q, added to this thread's sums
-        auto fs_op_add = [&](const FT *Q, int s) {
+        // the operators of a slice's coordinates, added to this thread's sums
+        auto fs_op_add = [&](const FT *x) {
             FT ov[FS_NOPS];
-            fs_ops(FS_ARGS_AT(Q, s), ov);
+            fs_ops(FS_ARGS_OF(x), ov);
 #pragma unroll
             for (int i = 0; i < FS_NOPS; i++) {
 #if FS_ACCUM == 0
@@ -881,10 +909,10 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
         };
 #endif
 #if FS_NCOR > 0
-        // the correlator values of slice s of path Q into the measurement's buffer C
-        auto fs_cor_put = [&](const FT *Q, int s) {
+        // the correlator values of slice s, coordinates x, into the measurement's buffer C
+        auto fs_cor_put = [&](const FT *x, int s) {
             FT cv[FS_NCOR];
-            fs_cors(FS_ARGS_AT(Q, s), cv);
+            fs_cors(FS_ARGS_OF(x), cv);
 #pragma unroll
             for (int c = 0; c < FS_NCOR; c++) {
                 C[c * FS_CSTRIDE + s] = cv[c];
@@ -1176,7 +1204,12 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
                 __syncthreads();
                 const FT *Q = SN0 + (run & 1) * FS_SNSTRIDE;
 #pragma unroll 1
-                for (int s = lt; s < FS_N; s += FS_CTPW) fs_cor_put(Q, s);
+                for (int s = lt; s < FS_N; s += FS_CTPW) {
+                    FT x[FS_DOF];
+#pragma unroll
+                    for (int d = 0; d < FS_DOF; d++) x[d] = FS_AT(Q, d, s);
+                    fs_cor_put(x, s);
+                }
                 asm volatile("bar.sync 2, %0;" ::"n"(FS_BLOCK - FS_MBLOCK) : "memory");
                 fs_cor_lags4(C);
             }
@@ -1198,7 +1231,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
                     const unsigned long long k = a.step_base + (unsigned long long)run * FS_MSTEPS + step;
 #endif
 #if FS_PATH_SHIFT
-                    n_acc += (fs_u32)fs_path_shift_move(P, k, is, fs, a.shift_old + (size_t)w * FS_N);
+                    n_acc += (fs_u32)fs_path_shift_move(P, k, is, fs, a.shift_old + w);
 #endif
 #if FS_SNM
                     n_acc += (fs_u32)fs_single_node_move(P, k, fs);
@@ -1264,43 +1297,52 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
             const int s_lo = 0, s_hi = FS_N;
 #endif
 #pragma unroll 1
-            for (int s = s_lo; s < (mover ? s_hi : s_lo); s++) {
+            for (int s0 = s_lo; s0 < (mover ? s_hi : s_lo); s0 += FS_MEAS_BATCH) {
+                FT xb[FS_MEAS_BATCH][FS_DOF];
+#pragma unroll
+                for (int b = 0; b < FS_MEAS_BATCH; b++)
+#pragma unroll
+                    for (int d = 0; d < FS_DOF; d++) xb[b][d] = FS_AT(P, d, s0 + b);
+#pragma unroll
+                for (int b = 0; b < FS_MEAS_BATCH; b++) {
+                    const int s = s0 + b;
+                    const FT *x = xb[b];
+                    (void)s;
 #if FS_NOPS > 0
-                fs_op_add(P, s);
+                    fs_op_add(x);
 #endif
 #if FS_PIPE
 #pragma unroll
-                for (int d = 0; d < FS_DOF; d++) FS_AT(SN, d, s) = FS_AT(P, d, s);
+                    for (int d = 0; d < FS_DOF; d++) FS_AT(SN, d, s) = x[d];
 #elif FS_NCOR > 0
-                fs_cor_put(P, s);
+                    fs_cor_put(x, s);
 #endif
 #if FS_BINS
-                {
-                    int ok = 1, inc = 1, bi = 0;
+                    {
+                        int ok = 1, inc = 1, bi = 0;
 #pragma unroll
-                    for (int d = 0; d < FS_DOF; d++) {
-                        const FT x = FS_AT(P, d, s);
-                        if (x < (FT)FS_XMIN || x >= (FT)FS_XMAX) ok = 0;
-                        bi += (int)((fs_u32)FS_MUL(FS_SUB(x, (FT)FS_XMIN), (FT)FS_INVBIN)) * inc;
-                        inc *= FS_BINRES;
+                        for (int d = 0; d < FS_DOF; d++) {
+                            if (x[d] < (FT)FS_XMIN || x[d] >= (FT)FS_XMAX) ok = 0;
+                            bi += (int)((fs_u32)FS_MUL(FS_SUB(x[d], (FT)FS_XMIN), (FT)FS_INVBIN)) * inc;
+                            inc *= FS_BINRES;
+                        }
+                        if (ok) atomicAdd(a.bins + bi, 1u);
                     }
-                    if (ok) atomicAdd(a.bins + bi, 1u);
-                }
 #endif
 #if FS_NHIST > 0
-                {
-                    FT hv[FS_NHIST];
-                    fs_hist(FS_ARGS_AT(P, s), hv);
+                    {
+                        FT hv[FS_NHIST];
+                        fs_hist(FS_ARGS_OF(x), hv);
 #pragma unroll
-                    for (int h = 0; h < FS_NHIST; h++) {
-                        const FT x = hv[h];
-                        if (x >= (FT)FS_HLO && x < (FT)FS_HHI) {
-                            const int b = (int)FS_MUL(FS_SUB(x, (FT)FS_HLO), (FT)FS_HINVW);
-                            if (b >= 0 && b < FS_HBINS) atomicAdd(s_hist + b, 1u);
+                        for (int h = 0; h < FS_NHIST; h++) {
+                            if (hv[h] >= (FT)FS_HLO && hv[h] < (FT)FS_HHI) {
+                                const int k = (int)FS_MUL(FS_SUB(hv[h], (FT)FS_HLO), (FT)FS_HINVW);
+                                if (k >= 0 && k < FS_HBINS) atomicAdd(s_hist + k, 1u);
+                            }
                         }
                     }
-                }
 #endif
+                }
             }
 #if FS_NOPS > 0
             if (mover) fs_op_flush();
