@@ -1481,6 +1481,49 @@ extern "C" int fs_get_walker_operators(fs_handle *h, double *out, size_t n)
     return FS_OK;
 }
 
+// The precision study's three columns (FP32, Kahan, FP64 sums) of the same means,
+// out[column][op][walker], FP64: one warp a walker, whose lanes read its threads' 24-byte
+// records side by side.  Bound by the launch and the read-back: 52 us for 4096 walkers of 256
+// work-items, where reading 25 MB of raw sums back and averaging them on the host took 13 ms.
+__global__ void fs_walker_ops_study_kernel(const double *ops, int n_walkers, int tpw, int wpg, int nwg, int nops,
+                                           int parallel, double *out)
+{
+    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) / 32), lane = threadIdx.x % 32;
+    if (w >= n_walkers) return;
+    const long long first = parallel ? (long long)(w / wpg) * tpw + (long long)(w % wpg) * nwg * tpw : w;
+    for (int op = 0; op < nops; op++) {
+        double s[3] = {0.0, 0.0, 0.0};
+        for (int t = lane; t < tpw; t += 32)
+#pragma unroll
+            for (int c = 0; c < 3; c++) s[c] += ops[((first + t) * nops + op) * 3 + c];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            for (int k = 16; k >= 1; k >>= 1) s[c] += __shfl_xor_sync(0xFFFFFFFFu, s[c], k);
+            if (lane == 0) out[((size_t)c * nops + op) * n_walkers + w] = s[c] / tpw;
+        }
+    }
+}
+
+extern "C" int fs_get_walker_operators_study(fs_handle *h, double *out, size_t n)
+{
+    if (!h || !out) return FS_ERR_CONFIG;
+    const fs_config &c = h->cfg;
+    const int nops = (int)h->ops.size();
+    if (c.accum != 3) return fail(h, FS_ERR_STATE, "the three columns are kept in study accumulation only");
+    if (n != (size_t)3 * nops * c.n_walkers)
+        return fail(h, FS_ERR_IO, "expected %zu values", (size_t)3 * nops * c.n_walkers);
+    if (nops == 0) return FS_OK;
+    CUDA_TRY(h, cudaSetDevice(h->device), FS_ERR_CUDA);
+    if (!h->d_wops) CUDA_TRY(h, cudaMalloc((void **)&h->d_wops, n * sizeof(double)), FS_ERR_OOM);
+    fs_walker_ops_study_kernel<<<(unsigned)(((size_t)c.n_walkers * 32 + 255) / 256), 256, 0, h->stream>>>(
+        (const double *)h->d_ops, c.n_walkers, h->tpw, c.walkers_per_group,
+        c.n_walkers / std::max(1, c.walkers_per_group), nops, c.enable_parallelize_path ? 1 : 0, h->d_wops);
+    CUDA_TRY(h, cudaGetLastError(), FS_ERR_LAUNCH);
+    CUDA_TRY(h, cudaMemcpyAsync(out, h->d_wops, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream), FS_ERR_CUDA);
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream), FS_ERR_LAUNCH);
+    return FS_OK;
+}
+
 extern "C" int fs_get_correlator(fs_handle *h, double *out, size_t n)
 {
     if (!h) return FS_ERR_CONFIG;

@@ -432,6 +432,11 @@ class PIMCKernel:
         if self._accumulation != "study":
             raise Exception("create the kernel with accumulation='study'")
         nops = len(self._operators)
+        if self._enableParallelizePath or self._nbrOfWalkersPerWorkGroup == 1:
+            # reduced on the device: the raw sums are 24 bytes per operator and work-item
+            out = np.empty((3, nops, self._nbrOfWalkers), np.float64)
+            check(lib().fs_get_walker_operators_study(self._handle, out.ctypes.data, out.size), self._handle)
+            return out
         raw = self._raw_operators().reshape(self._nbrOfThreads, nops, 3)
         return np.stack([self._per_walker(raw[:, :, k]).T for k in range(3)])
 

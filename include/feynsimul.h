@@ -238,6 +238,9 @@ int fs_get_correlator(fs_handle *h, double *out, size_t n);
  * device in FP64 (the fixed-mode reduction of PIMCKernel.getOperators, kernel.py:576-606).
  * Not for FS_ACCUM_STUDY. */
 int fs_get_walker_operators(fs_handle *h, double *out, size_t n);
+/* The same for FS_ACCUM_STUDY: [3][n_ops][walkers], the means of the FP32, Kahan and FP64
+ * sums. */
+int fs_get_walker_operators_study(fs_handle *h, double *out, size_t n);
 int fs_get_accepts(fs_handle *h, uint32_t *out, size_t n);
 int fs_get_bins(fs_handle *h, uint32_t *out, size_t n);
 int fs_get_histogram(fs_handle *h, uint64_t *out, size_t n);
