@@ -9,10 +9,9 @@
 // (largest first, so the ragged tail is short) and run all the launch's sweeps on the
 // tile: the same Metropolis-bisection move as fs_pimc.cuh (kernel.c:258-399, with the
 // fixed-mode xorshift or RANLUX streams), but N, S, epsilon, the bisection widths and the walker
-// counts are runtime values of the system, the path tile lives in shared memory while the
-// saved old segments go to the CTA's slice of a global scratch buffer (a 27-DOF,
-// 1024-slice walker's path alone takes 117 KB), and a walker wider than a warp
-// synchronises with a named barrier of its own.
+// counts are runtime values of the system, the path tile lives in shared memory (saved old
+// segments in registers, or in the CTA's slice of a global scratch buffer where they are too
+// large), and a walker wider than a warp synchronises with a named barrier of its own.
 #pragma once
 
 #define FS_BATCH_MAX_S 10
@@ -71,6 +70,17 @@ __device__ __forceinline__ void fs_walker_sync(int tpw, int wl)
     }
 }
 
+// Shared-memory path layout: slice s of a degree of freedom at (s mod 2^S) * T + s / 2^S, the
+// potential cache's order.  The segment threads, whose slices lie 2^S apart, touch consecutive
+// words, so there are no bank conflicts and no padding: a thread of S = 2 and 27 degrees of
+// freedom takes 432 bytes (540 with a padding word every 2^S slices) and a 10-atom tile of 512
+// threads fits an SM.  Walkers of fewer than 32 threads continue the sequence of words modulo 32.
+__host__ __device__ __forceinline__ int fs_batch_wstride(int dof, int N, int tpw)
+{
+    const int words = dof * N;
+    return tpw >= 32 ? words : words + (tpw - words % 32 + 32) % 32;
+}
+
 // One tile: walkers [tile*wpb, ...) of system sd.  All threads of the CTA call it.
 // Systems of 3 or more DOF keep V of every slice in device memory between moves (as the
 // sweep's potential cache: slice s of a walker at (s mod 2^S) * (N / 2^S) + s / 2^S, so a
@@ -81,15 +91,22 @@ __device__ __forceinline__ void fs_walker_sync(int tpw, int wl)
 // GLOBAL: the walkers' paths stay in device memory (L1/L2) and are worked on in place, for
 // walkers too large to put enough of them in shared memory to fill the CTA (the same
 // arithmetic as the shared-memory tile, like the sweep's global-path mode).
-template <int DOF, class Sys, bool GLOBAL>
+// SC: the bisection level as a constant, 0 for levels above 4.  A constant level keeps the old
+// segment in registers where it is at most 112 values (the register budget is 128); otherwise
+// it goes to the CTA's slice of the scratch buffer.
+// What bounds a tile is its 16 warps' instruction issue and latency.  24 clusters of 3 to 10 atoms,
+// N = 128..1024, 512 threads, us a launch: 979 with padded paths of 200 KB at most (10-atom tiles
+// of 256 to 320 threads) and scratch segments, 739 with this layout and registers; a 32-system
+// sample of 2048 walkers each 8181 -> 6772 (6.81 -> 8.22e9 node updates/s).
+template <int DOF, int SC, class Sys, bool GLOBAL>
 __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, float *smem, size_t old_slot_floats)
 {
     const int tid = threadIdx.x;
-    const int N = sd.N, S = sd.S, seg = 1 << S, tpw = sd.tpw;
-    const int dstride = N + (N >> S);
-    int wstride = DOF * dstride;
-    wstride = ((wstride + 15) / 16) * 16;
-    if ((wstride / 16) % 2 == 0) wstride += 16;
+    const int N = sd.N, S = SC > 0 ? SC : sd.S, seg = 1 << S, tpw = sd.tpw;
+    constexpr bool VC = DOF >= 3;
+    constexpr int NODES = SC > 0 ? (1 << SC) - 1 : 1;
+    constexpr bool REGS = SC > 0 && NODES * (DOF + (VC ? 1 : 0)) <= 112;
+    const int wstride = fs_batch_wstride(DOF, N, tpw);
     const int w0 = tile * sd.wpb;
     const int n_here = min(sd.wpb, sd.n_walkers - w0);
     const int wl = tid / tpw, t = tid % tpw;
@@ -97,11 +114,11 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
     const int nthr = sd.wpb * tpw;
     // saved old segments: this CTA's slice of the global scratch, [(seg-1)*DOF][tile threads]
     float *s_old = sd.old_scratch + (size_t)blockIdx.x * old_slot_floats;
-    double *s_op = (double *)(GLOBAL ? smem : smem + sd.wpb * wstride);  // [wpb][nops]
-    constexpr bool VC = DOF >= 3;
+    double *s_op = (double *)(GLOBAL ? smem : smem + (sd.wpb * wstride + 1) / 2 * 2);  // [wpb][nops]
     float *s_oldv = s_old + (size_t)(seg - 1) * DOF * nthr;  // [(seg-1)][tile threads]
 
-#define FSB_AT(P, d, s) (GLOBAL ? (P)[(d) * N + (s)] : (P)[(d) * dstride + (s) + ((s) >> S)])
+#define FSB_IDX(s) ((((s) & (seg - 1)) * tpw) + ((s) >> S))
+#define FSB_AT(P, d, s) ((P)[(d) * N + (GLOBAL ? (s) : FSB_IDX(s))])
     {
         if (!GLOBAL) {
             const size_t base = (size_t)w0 * DOF * N;
@@ -135,14 +152,13 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
 #endif
         }
         float *Vc = VC ? sd.vcache + (size_t)w * N : nullptr;
-#define FSB_VIDX(s) ((((s) & (seg - 1)) * tpw) + ((s) >> S))
         if (VC) {
 #pragma unroll 1
             for (int s = t * seg; s < (t + 1) * seg; s++) {
                 float x[DOF];
 #pragma unroll
                 for (int d = 0; d < DOF; d++) x[d] = FSB_AT(P, d, s);
-                Vc[FSB_VIDX(s)] = Sys::pot(x);
+                Vc[FSB_IDX(s)] = Sys::pot(x);
             }
             fs_walker_sync(tpw, wl);
         }
@@ -160,22 +176,43 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
                 // ---- bisection move (kernel.c:258-399) ----
                 float aOld = 0.f, aNew = 0.f;
                 float x[DOF];
-#pragma unroll 1
-                for (int i = 1; i < seg; i++) {
-                    const int p = (start + i) & (N - 1);
+                float old[REGS ? NODES * DOF : 1], oldv[REGS && VC ? NODES : 1];
+                if (REGS) {
 #pragma unroll
-                    for (int d = 0; d < DOF; d++) {
-                        x[d] = FSB_AT(P, d, p);
-                        s_old[((i - 1) * DOF + d) * nthr + tid] = x[d];
+                    for (int i = 1; i <= NODES; i++) {
+                        const int p = (start + i) & (N - 1);
+#pragma unroll
+                        for (int d = 0; d < DOF; d++) old[(REGS ? i - 1 : 0) * DOF + (REGS ? d : 0)] = FSB_AT(P, d, p);
                     }
-                    if (!VC) aOld = __fadd_rn(aOld, __fmul_rn(eps, Sys::pot(x)));
-                }
-                if (VC) {
-#pragma unroll 4
-                    for (int i = 1; i < seg; i++) {
-                        const float v = Vc[FSB_VIDX((start + i) & (N - 1))];
-                        s_oldv[(i - 1) * nthr + tid] = v;
+#pragma unroll
+                    for (int i = 1; i <= NODES; i++) {
+                        float v;
+                        if (VC) {
+                            v = Vc[FSB_IDX((start + i) & (N - 1))];
+                            oldv[REGS && VC ? i - 1 : 0] = v;
+                        } else {
+                            v = Sys::pot(old + (REGS ? (i - 1) * DOF : 0));
+                        }
                         aOld = __fadd_rn(aOld, __fmul_rn(eps, v));
+                    }
+                } else {
+#pragma unroll 1
+                    for (int i = 1; i < seg; i++) {
+                        const int p = (start + i) & (N - 1);
+#pragma unroll
+                        for (int d = 0; d < DOF; d++) {
+                            x[d] = FSB_AT(P, d, p);
+                            s_old[((i - 1) * DOF + d) * nthr + tid] = x[d];
+                        }
+                        if (!VC) aOld = __fadd_rn(aOld, __fmul_rn(eps, Sys::pot(x)));
+                    }
+                    if (VC) {
+#pragma unroll 4
+                        for (int i = 1; i < seg; i++) {
+                            const float v = Vc[FSB_IDX((start + i) & (N - 1))];
+                            s_oldv[(i - 1) * nthr + tid] = v;
+                            aOld = __fadd_rn(aOld, __fmul_rn(eps, v));
+                        }
                     }
                 }
 #pragma unroll 1
@@ -207,16 +244,26 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
 #pragma unroll
                     for (int d = 0; d < DOF; d++) x[d] = FSB_AT(P, d, p);
                     const float v = Sys::pot(x);
-                    if (VC) Vc[FSB_VIDX(p)] = v;
+                    if (VC) Vc[FSB_IDX(p)] = v;
                     aNew = __fadd_rn(aNew, __fmul_rn(eps, v));
                 }
                 if (__expf(__fsub_rn(aOld, aNew)) < fsb_uniform(g)) {
-#pragma unroll 1
-                    for (int i = 1; i < seg; i++) {
-                        const int p = (start + i) & (N - 1);
+                    if (REGS) {
 #pragma unroll
-                        for (int d = 0; d < DOF; d++) FSB_AT(P, d, p) = s_old[((i - 1) * DOF + d) * nthr + tid];
-                        if (VC) Vc[FSB_VIDX(p)] = s_oldv[(i - 1) * nthr + tid];
+                        for (int i = 1; i <= NODES; i++) {
+                            const int p = (start + i) & (N - 1);
+#pragma unroll
+                            for (int d = 0; d < DOF; d++) FSB_AT(P, d, p) = old[(REGS ? i - 1 : 0) * DOF + (REGS ? d : 0)];
+                            if (VC) Vc[FSB_IDX(p)] = oldv[REGS && VC ? i - 1 : 0];
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int i = 1; i < seg; i++) {
+                            const int p = (start + i) & (N - 1);
+#pragma unroll
+                            for (int d = 0; d < DOF; d++) FSB_AT(P, d, p) = s_old[((i - 1) * DOF + d) * nthr + tid];
+                            if (VC) Vc[FSB_IDX(p)] = s_oldv[(i - 1) * nthr + tid];
+                        }
                     }
                 } else {
                     n_acc++;
@@ -269,6 +316,6 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
         for (int i = tid; i < n_here * sd.nops; i += blockDim.x) sd.op_sums[(size_t)w0 * sd.nops + i] += s_op[i];
     }
     __syncthreads();  // the next tile reuses the shared-memory tile
-#undef FSB_VIDX
+#undef FSB_IDX
 #undef FSB_AT
 }

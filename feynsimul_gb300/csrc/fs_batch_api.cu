@@ -78,14 +78,16 @@ static int bfail(int code, const char *fmt, ...)
         if (e_ != cudaSuccess) return bfail(FS_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
+// shared memory of a tile of wpb walkers (fs_batch_wstride in fs_batch.cuh)
 static size_t tile_smem_bytes(int dof, int N, int S, int wpb, int nops)
 {
-    long long dstride = N + (N >> S);
-    long long wstride = (long long)dof * dstride;
-    wstride = ((wstride + 15) / 16) * 16;
-    if ((wstride / 16) % 2 == 0) wstride += 16;
-    return (size_t)(wpb * wstride) * 4 + (size_t)wpb * std::max(nops, 1) * 8;
+    const long long tpw = N >> S, words = (long long)dof * N;
+    const long long wstride = tpw >= 32 ? words : words + (tpw - words % 32 + 32) % 32;
+    return (size_t)((wpb * wstride + 1) / 2 * 2) * 4 + (size_t)wpb * std::max(nops, 1) * 8;
 }
+
+// a tile's most: an SM's 227 KB less the kernel's static shared memory
+static const size_t kTileSmem = 226 * 1024;
 
 static void free_batch(fs_batch *b)
 {
@@ -152,6 +154,12 @@ extern "C" int fs_batch_create(int32_t n_types, const int32_t *type_dof, const c
     b->type_dof.assign(type_dof, type_dof + n_types);
     b->sys.assign(systems, systems + n_systems);
     size_t max_smem = 0, max_old = 0;
+    std::vector<char> given;  // systems whose walkers per tile the caller chose
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+        sms = 152;
+    cudaGetLastError();
     for (int i = 0; i < n_systems; i++) {
         fs_batch_system &s = b->sys[i];
         if (s.type < 0 || s.type >= n_types) { free_batch(b); return bfail(FS_ERR_CONFIG, "system %d: bad type", i); }
@@ -168,27 +176,71 @@ extern "C" int fs_batch_create(int32_t n_types, const int32_t *type_dof, const c
             free_batch(b);
             return bfail(FS_ERR_CONFIG, "system %d: N / 2^S = %d threads per walker does not fit the block", i, tpw);
         }
-        int wpb_max = std::min(s.walkers_per_tile > 0 ? s.walkers_per_tile : block_threads, block_threads / tpw);
-        if (tpw > 32) wpb_max = std::min(wpb_max, 15);  // named barriers 1..15
-        int wpb = wpb_max;
-        while (wpb > 1 && tile_smem_bytes(dof, s.n_slices, s.bisection_level, wpb, n_ops) > 200 * 1024) wpb--;
-        // walkers so large that shared memory holds too few of them to fill half the CTA
-        // (large clusters at N = 1024) work on their paths in device memory instead
-        const bool global = wpb * tpw * 2 < block_threads && dof > 8;
-        size_t tile_bytes;
-        if (global) {
-            wpb = wpb_max;
-            tile_bytes = (size_t)wpb * std::max(n_ops, 1) * 8;
-        } else {
-            tile_bytes = tile_smem_bytes(dof, s.n_slices, s.bisection_level, wpb, n_ops);
-            if (tile_bytes > 220 * 1024) {
-                free_batch(b);
-                return bfail(FS_ERR_CONFIG, "system %d: one walker's path does not fit in shared memory", i);
-            }
+    }
+    // walkers per tile of system i with `budget` bytes of shared memory a CTA, and whether its
+    // walkers are so large that shared memory holds too few of them to fill half the CTA (large
+    // clusters at N = 1024): those work on their paths in device memory instead
+    auto place = [&](int i, size_t budget, bool *global) {
+        const fs_batch_system &s = b->sys[i];
+        const int dof = b->type_dof[s.type], tpw = s.n_slices >> s.bisection_level;
+        int most = std::min(s.walkers_per_tile > 0 ? s.walkers_per_tile : block_threads, block_threads / tpw);
+        if (tpw > 32) most = std::min(most, 15);  // named barriers 1..15
+        int wpb = most;
+        if (s.walkers_per_tile > 0) budget = kTileSmem;
+        while (wpb > 1 && tile_smem_bytes(dof, s.n_slices, s.bisection_level, wpb, n_ops) > budget) wpb--;
+        *global = wpb * tpw * 2 < block_threads && dof > 8;
+        return *global ? most : wpb;
+    };
+    // CTAs per SM: 512 threads at the kernel's 128 registers, so a smaller CTA leaves shared memory
+    // for others, unless that sends a system to device memory or has no room for a walker (24
+    // clusters of 3 to 10 atoms, 256 threads, 32 a walker: one CTA per SM 1325 us a launch, two
+    // 1076; 16 a walker, where two CTAs would move paths to device memory: 1551 against 2507)
+    int per_sm = std::max(1, 512 / block_threads);
+    auto budget_of = [&](int k) { return k == 1 ? kTileSmem : (size_t)227 * 1024 / k - 2048; };
+    for (bool fits = false; per_sm > 1 && !fits; per_sm = fits ? per_sm : per_sm / 2) {
+        fits = true;
+        for (int i = 0; i < n_systems && fits; i++) {
+            const fs_batch_system &s = b->sys[i];
+            bool full = false, part = false;
+            place(i, kTileSmem, &full);
+            const int wpb = place(i, budget_of(per_sm), &part);
+            fits = part ? full
+                        : tile_smem_bytes(b->type_dof[s.type], s.n_slices, s.bisection_level, wpb, n_ops) <=
+                              budget_of(per_sm);
+        }
+    }
+    for (int i = 0; i < n_systems; i++) {
+        fs_batch_system &s = b->sys[i];
+        bool global = false;
+        const int wpb = place(i, budget_of(per_sm), &global);
+        if (!global && tile_smem_bytes(b->type_dof[s.type], s.n_slices, s.bisection_level, wpb, n_ops) > kTileSmem) {
+            free_batch(b);
+            return bfail(FS_ERR_CONFIG, "system %d: one walker's path does not fit in shared memory", i);
         }
         b->sys_global.push_back(global ? 1 : 0);
+        given.push_back(s.walkers_per_tile > 0);
         s.walkers_per_tile = wpb;
-        max_smem = std::max(max_smem, tile_bytes);
+    }
+    // few walkers: tiles of fewer walkers, down to a warp of threads, until every CTA has one (40
+    // walkers each of 6 small clusters, 256 threads: 18 tiles 303 us a launch, 120 tiles 132)
+    for (bool more = true; more;) {
+        more = false;
+        long long tiles = 0;
+        for (const fs_batch_system &s : b->sys) tiles += (s.n_walkers + s.walkers_per_tile - 1) / s.walkers_per_tile;
+        for (int i = 0; i < n_systems && tiles < (long long)sms * per_sm; i++) {
+            fs_batch_system &s = b->sys[i];
+            const int wpb = s.walkers_per_tile, half = (wpb + 1) / 2;
+            if (given[i] || wpb == 1 || half * (s.n_slices >> s.bisection_level) < 32) continue;
+            tiles += (s.n_walkers + half - 1) / half - (s.n_walkers + wpb - 1) / wpb;
+            s.walkers_per_tile = half;
+            more = true;
+        }
+    }
+    for (int i = 0; i < n_systems; i++) {
+        const fs_batch_system &s = b->sys[i];
+        const int dof = b->type_dof[s.type], tpw = s.n_slices >> s.bisection_level, wpb = s.walkers_per_tile;
+        max_smem = std::max(max_smem, b->sys_global[i] ? (size_t)wpb * std::max(n_ops, 1) * 8
+                                                       : tile_smem_bytes(dof, s.n_slices, s.bisection_level, wpb, n_ops));
         const size_t seg = (size_t)1 << s.bisection_level;
         // saved segment, and with the potential cache (3 or more DOF) its cached values
         max_old = std::max(max_old, (seg - 1) * (dof + (dof >= 3 ? 1 : 0)) * (size_t)(wpb * tpw));
@@ -240,15 +292,16 @@ extern "C" int fs_batch_create(int32_t n_types, const int32_t *type_dof, const c
          "        if (it >= n_items) break;\n"
          "        const FsBatchItem item = items[it];\n"
          "        const FsBatchSys &sd = sys[item.sys];\n"
-         "        switch (sd.type * 2 + sd.global) {\n";
-    // one case per (type, path placement) pair the batch uses
-    std::vector<char> used(2 * n_types, 0);
-    for (int i = 0; i < n_systems; i++) used[2 * b->sys[i].type + b->sys_global[i]] = 1;
-    for (int k = 0; k < n_types; k++)
-        for (int g = 0; g < 2; g++)
-            if (used[2 * k + g])
-                o << "        case " << (2 * k + g) << ": fs_batch_tile<" << b->type_dof[k] << ", fs_type_" << k
-                  << "::Sys, " << (g ? "true" : "false") << ">(sd, item.tile, fsb_smem, old_slot); break;\n";
+         "        switch ((sd.type * 2 + sd.global) * 5 + (sd.S <= 4 ? sd.S : 0)) {\n";
+    // one case per (type, path placement, level) the batch uses; levels above 4 share one
+    std::vector<char> used(10 * n_types, 0);
+    auto level = [&](int i) { return b->sys[i].bisection_level <= 4 ? b->sys[i].bisection_level : 0; };
+    for (int i = 0; i < n_systems; i++) used[(2 * b->sys[i].type + b->sys_global[i]) * 5 + level(i)] = 1;
+    for (int k = 0; k < 10 * n_types; k++)
+        if (used[k])
+            o << "        case " << k << ": fs_batch_tile<" << b->type_dof[k / 10] << ", " << k % 5 << ", fs_type_"
+              << k / 10 << "::Sys, " << (k / 5 % 2 ? "true" : "false")
+              << ">(sd, item.tile, fsb_smem, old_slot); break;\n";
     o << "        default: break;\n        }\n    }\n}\n";
     b->source = o.str();
     std::string cubin;
