@@ -10,6 +10,7 @@
 #include <nvrtc.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cctype>
 #include <chrono>
 #include <cmath>
@@ -100,8 +101,16 @@ struct fs_handle {
     uint32_t *d_rtab = nullptr, *d_gtab = nullptr, *d_bins = nullptr;
     void *d_ops = nullptr, *d_cor = nullptr;
     unsigned long long *d_hist = nullptr;
-    int *d_status = nullptr;   // [0] FS_STATUS_* flags, [1] 1 + a walker that raised one
-    bool status_pending = false;  // a sweep ran since fs_sync last read d_status
+    // Page-locked host memory that kernels write and this library reads once the stream has
+    // drained (see host_results): the status word ([0] FS_STATUS_* flags, [1] 1 + a walker that
+    // raised one), and where they fit the accepts, the per-walker operator means and the
+    // correlator moments
+    void *pinned = nullptr;
+    int *status = nullptr;
+    uint32_t *h_accepts = nullptr;
+    double *h_wops = nullptr, *h_red = nullptr;
+    std::atomic<bool> idle{true};  // nothing was queued since the stream last drained
+    bool status_pending = false;   // a sweep ran since fs_sync last read the status word
     void *d_mlp_frag = nullptr;
     float *d_mlp_bias = nullptr;
     double mlp_inv_scale = 1.0;
@@ -649,10 +658,49 @@ static int validate(const fs_config &c, int nops, int ncor, int nhist)
 static void free_buffers(fs_handle *h)
 {
     void *bufs[] = {h->d_paths, h->d_accepts, h->d_seeds, h->d_snap, h->d_wseeds, h->d_rtab,
-                    h->d_gtab, h->d_bins, h->d_ops, h->d_cor, h->d_hist, h->d_status,
+                    h->d_gtab, h->d_bins, h->d_ops, h->d_cor, h->d_hist,
                     h->d_mlp_frag, h->d_mlp_bias, h->d_red, h->d_shift_old, h->d_wops, h->d_vcache};
     for (void *p : bufs)
-        if (p) cudaFree(p);
+        if (p && p != h->h_accepts) cudaFree(p);
+    if (h->pinned) cudaFreeHost(h->pinned);
+}
+
+// Results a run loop reads after every launch are small, and a device-to-host copy with its
+// synchronisation takes 10 us or more whatever its size.  So the kernels write them to page-locked
+// host memory, and a getter on a drained stream is a memcpy: one block per handle, each part at
+// most 128 KB (64 oscillators, a run with operators, accepts and paths read: 84 -> 58 us).  Larger
+// results stay in device memory: a copy of 1 MB takes 20 us, the memcpy 68.
+static const size_t kHostResult = 128 * 1024;
+static int host_results(fs_handle *h, size_t accepts, size_t wops, size_t red)
+{
+    auto part = [](size_t bytes) { return bytes <= kHostResult ? (bytes + 255) / 256 * 256 : 0; };
+    const size_t bytes = 256 + part(accepts) + part(wops) + part(red);
+    cudaError_t e = cudaHostAlloc(&h->pinned, bytes, cudaHostAllocMapped);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        h->pinned = nullptr;
+        return fail(h, FS_ERR_OOM, "Unable to allocate page-locked host memory (%zu bytes: %s)", bytes,
+                    cudaGetErrorString(e));
+    }
+    memset(h->pinned, 0, bytes);
+    char *at = (char *)h->pinned;
+    h->status = (int *)at;
+    at += 256;
+    if (part(accepts)) h->h_accepts = (uint32_t *)at;
+    at += part(accepts);
+    if (part(wops)) h->h_wops = (double *)at;
+    at += part(wops);
+    if (part(red)) h->h_red = (double *)at;
+    return FS_OK;
+}
+
+// the handle's stream drained: everything queued before has run
+static cudaError_t drain(fs_handle *h)
+{
+    if (h->idle) return cudaSuccess;
+    cudaError_t e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess) h->idle = true;
+    return e;
 }
 
 static int dalloc(fs_handle *h, void **p, size_t bytes)
@@ -957,7 +1005,10 @@ extern "C" int fs_create(const fs_config *cfg, const char *potential, const char
         return FS_ERR_OOM;
     }
     CREATE_TRY(dalloc(h, &h->d_paths, W * c.dof * N * h->ft));
-    CREATE_TRY(dalloc(h, (void **)&h->d_accepts, T * 4));
+    CREATE_TRY(host_results(h, T * 4, W * h->ops.size() * (c.accum == 3 ? 3 : 1) * 8,
+                            h->cors.size() * (N / 2) * (c.accum == 3 ? 3 : 1) * 16));
+    if (h->h_accepts) h->d_accepts = h->h_accepts;
+    else CREATE_TRY(dalloc(h, (void **)&h->d_accepts, T * 4));
     if (c.enable_ranlux) {
         CREATE_TRY(dalloc(h, (void **)&h->d_rtab, T * 112));
         CREATE_TRY(dalloc(h, (void **)&h->d_gtab, h->g_rows * 112));
@@ -970,7 +1021,6 @@ extern "C" int fs_create(const fs_config *cfg, const char *potential, const char
     CREATE_TRY(dalloc(h, &h->d_cor, h->n_cor_lags * h->cor_elem));
     CREATE_TRY(dalloc(h, (void **)&h->d_bins, h->n_bins * 4));
     CREATE_TRY(dalloc(h, (void **)&h->d_hist, h->n_hist * 8));
-    CREATE_TRY(dalloc(h, (void **)&h->d_status, 16));
     if ((c.moves & FS_MOVE_PATH_SHIFT) && !c.compat) CREATE_TRY(dalloc(h, &h->d_shift_old, W * N * h->ft));
     if (h->vglobal) CREATE_TRY(dalloc(h, &h->d_vcache, W * N * h->ft));
     if (c.learned) {
@@ -1180,6 +1230,7 @@ extern "C" int fs_run(fs_handle *h, int32_t n_launches)
     FsArgsHost a;
     fill_args(h, a);
     void *args[] = {&a};
+    h->idle = false;
     CUDA_TRY(h, cudaEventRecord(h->ev0, h->stream), FS_ERR_CUDA);
     for (int i = 0; i < n_launches; i++) {
         a.step_base = h->steps_done;  // copied at launch
@@ -1222,6 +1273,7 @@ extern "C" int fs_run_host(fs_handle *h, const void *paths_in, void *paths_out, 
         const long long half_wave = std::max(1ll, (long long)h->resident_per_sm * device_sms() / 2);
         n_chunks = (int)std::max(1ll, std::min(4ll, (long long)h->grid / half_wave));
     }
+    h->idle = false;
     if (h->d_snap) n_chunks = 1;
     n_chunks = std::min(n_chunks, std::min(h->grid, 64));
     h->last_chunks = n_chunks;
@@ -1356,7 +1408,7 @@ static void fill_args(fs_handle *h, FsArgsHost &a)
     a.cor_means = h->d_cor;
     a.bins = h->d_bins;
     a.hist = h->d_hist;
-    a.status = h->d_status;
+    a.status = h->status;
     a.opnorm = 1.0 / ((double)c.operator_runs * c.n_slices * c.n_walkers / (double)h->n_threads);
     a.mlp_frag = h->d_mlp_frag;
     a.mlp_bias = h->d_mlp_bias;
@@ -1372,23 +1424,20 @@ static void fill_args(fs_handle *h, FsArgsHost &a)
 static int check_status(fs_handle *h)
 {
     if (!h->status_pending) return FS_OK;
-    int st[2] = {0, 0};
-    CUDA_TRY(h, cudaMemcpyAsync(st, h->d_status, sizeof st, cudaMemcpyDeviceToHost, h->stream), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream), FS_ERR_LAUNCH);
     h->status_pending = false;
-    if (!st[0]) return FS_OK;
-    CUDA_TRY(h, cudaMemsetAsync(h->d_status, 0, sizeof st, h->stream), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream), FS_ERR_LAUNCH);
+    const int flags = h->status[0], walker = h->status[1];
+    if (!flags) return FS_OK;
+    h->status[0] = h->status[1] = 0;
     return fail(h, FS_ERR_NUMERIC,
                 "walker %d: a path value is not finite (NaN or infinity) after the sweep; the paths and the "
-                "operator, correlator and histogram sums of this run are not usable", st[1] - 1);
+                "operator, correlator and histogram sums of this run are not usable", walker - 1);
 }
 
 extern "C" int fs_sync(fs_handle *h)
 {
     if (!h) return FS_ERR_CONFIG;
     CUDA_TRY(h, cudaSetDevice(h->device), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream), FS_ERR_LAUNCH);
+    CUDA_TRY(h, drain(h), FS_ERR_LAUNCH);
     return check_status(h);
 }
 
@@ -1400,7 +1449,10 @@ extern "C" int fs_sync_timeout(fs_handle *h, double seconds)
     auto t0 = std::chrono::steady_clock::now();
     for (;;) {
         cudaError_t e = cudaStreamQuery(h->stream);
-        if (e == cudaSuccess) return check_status(h);
+        if (e == cudaSuccess) {
+            h->idle = true;
+            return check_status(h);
+        }
         if (e != cudaErrorNotReady) return fail(h, FS_ERR_LAUNCH, "stream error: %s", cudaGetErrorString(e));
         double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (el > seconds)
@@ -1439,6 +1491,19 @@ extern "C" int fs_get_operators(fs_handle *h, double *out, size_t n)
     return FS_OK;
 }
 
+// n values that kernels of the handle's stream wrote to src (host or device memory), to out
+static int result_out(fs_handle *h, double *out, const double *src, size_t n, bool on_host)
+{
+    if (on_host) {
+        CUDA_TRY(h, cudaStreamSynchronize(h->stream), FS_ERR_LAUNCH);
+        memcpy(out, src, n * sizeof(double));
+        return FS_OK;
+    }
+    CUDA_TRY(h, cudaMemcpyAsync(out, src, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream), FS_ERR_CUDA);
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream), FS_ERR_LAUNCH);
+    return FS_OK;
+}
+
 // per-walker operator means: the mean over the walker's own threads of their per-thread
 // means (thread ids as in the sweep, kernel.c:539-541), FP64, out[op][walker]
 template <class T>
@@ -1465,20 +1530,20 @@ extern "C" int fs_get_walker_operators(fs_handle *h, double *out, size_t n)
     if (c.accum == 3) return fail(h, FS_ERR_STATE, "study accumulation keeps three columns: use fs_get_operators");
     if (nops == 0) return FS_OK;
     CUDA_TRY(h, cudaSetDevice(h->device), FS_ERR_CUDA);
-    if (!h->d_wops) CUDA_TRY(h, cudaMalloc((void **)&h->d_wops, n * sizeof(double)), FS_ERR_OOM);
+    double *dst = h->h_wops;
+    if (!dst && !h->d_wops) CUDA_TRY(h, cudaMalloc((void **)&h->d_wops, n * sizeof(double)), FS_ERR_OOM);
+    if (!dst) dst = h->d_wops;
     const unsigned grid = (unsigned)((n + 255) / 256);
     const int par = c.enable_parallelize_path ? 1 : 0;
     const int nwg = c.n_walkers / std::max(1, c.walkers_per_group);
     if (h->op_elem == 8)
         fs_walker_ops_kernel<double><<<grid, 256, 0, h->stream>>>((const double *)h->d_ops, c.n_walkers, h->tpw,
-                                                                  c.walkers_per_group, nwg, nops, par, h->d_wops);
+                                                                  c.walkers_per_group, nwg, nops, par, dst);
     else
         fs_walker_ops_kernel<float><<<grid, 256, 0, h->stream>>>((const float *)h->d_ops, c.n_walkers, h->tpw,
-                                                                 c.walkers_per_group, nwg, nops, par, h->d_wops);
+                                                                 c.walkers_per_group, nwg, nops, par, dst);
     CUDA_TRY(h, cudaGetLastError(), FS_ERR_LAUNCH);
-    CUDA_TRY(h, cudaMemcpyAsync(out, h->d_wops, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream), FS_ERR_LAUNCH);
-    return FS_OK;
+    return result_out(h, out, dst, n, dst == h->h_wops);
 }
 
 // The precision study's three columns (FP32, Kahan, FP64 sums) of the same means,
@@ -1514,14 +1579,14 @@ extern "C" int fs_get_walker_operators_study(fs_handle *h, double *out, size_t n
         return fail(h, FS_ERR_IO, "expected %zu values", (size_t)3 * nops * c.n_walkers);
     if (nops == 0) return FS_OK;
     CUDA_TRY(h, cudaSetDevice(h->device), FS_ERR_CUDA);
-    if (!h->d_wops) CUDA_TRY(h, cudaMalloc((void **)&h->d_wops, n * sizeof(double)), FS_ERR_OOM);
+    double *dst = h->h_wops;
+    if (!dst && !h->d_wops) CUDA_TRY(h, cudaMalloc((void **)&h->d_wops, n * sizeof(double)), FS_ERR_OOM);
+    if (!dst) dst = h->d_wops;
     fs_walker_ops_study_kernel<<<(unsigned)(((size_t)c.n_walkers * 32 + 255) / 256), 256, 0, h->stream>>>(
         (const double *)h->d_ops, c.n_walkers, h->tpw, c.walkers_per_group,
-        c.n_walkers / std::max(1, c.walkers_per_group), nops, c.enable_parallelize_path ? 1 : 0, h->d_wops);
+        c.n_walkers / std::max(1, c.walkers_per_group), nops, c.enable_parallelize_path ? 1 : 0, dst);
     CUDA_TRY(h, cudaGetLastError(), FS_ERR_LAUNCH);
-    CUDA_TRY(h, cudaMemcpyAsync(out, h->d_wops, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream), FS_ERR_LAUNCH);
-    return FS_OK;
+    return result_out(h, out, dst, n, dst == h->h_wops);
 }
 
 extern "C" int fs_get_correlator(fs_handle *h, double *out, size_t n)
@@ -1552,7 +1617,12 @@ extern "C" int fs_get_correlator(fs_handle *h, double *out, size_t n)
 extern "C" int fs_get_accepts(fs_handle *h, uint32_t *out, size_t n)
 {
     if (!h) return FS_ERR_CONFIG;
-    return copy_out(h, out, h->d_accepts, n * 4, (size_t)h->n_threads * 4);
+    if (!h->h_accepts) return copy_out(h, out, h->d_accepts, n * 4, (size_t)h->n_threads * 4);
+    if (n != (size_t)h->n_threads)
+        return fail(h, FS_ERR_IO, "buffer has %zu bytes, expected %zu", n * 4, (size_t)h->n_threads * 4);
+    CUDA_TRY(h, drain(h), FS_ERR_LAUNCH);
+    memcpy(out, h->h_accepts, n * 4);
+    return FS_OK;
 }
 extern "C" int fs_get_bins(fs_handle *h, uint32_t *out, size_t n)
 {
@@ -1587,43 +1657,85 @@ extern "C" int fs_set_correlator(fs_handle *h, const double *in, size_t n)
 }
 
 // ---- correlator moments over a walker range, on the device ----
-// Block b reduces walkers [w0 + b*chunk, ...) for every lag (threads stride the lags, so
-// a warp reads consecutive lags of one walker) and adds its partial sums atomically.
+// Stage 1: block b sums its share of the walkers for every lag and column (sum and sum of squares,
+// FP64) into one row of `part`; a warp reads consecutive lags of one walker, and where there are
+// fewer lags than threads the block takes several walkers at a time.  Stage 2 adds the rows.  No
+// atomics, so equal sums give equal bits, and nothing to clear.  Bound by its two launches:
+// 1024 walkers of 64 lags, with the read-back, 63 us before (a clear, atomics, two copies), 36 now.
+#define FS_MOM_THREADS 256
 template <int KIND>  // 0: float, 1: double, 2: study struct (3 columns)
-__global__ void fs_cor_moments_kernel(const unsigned char *cor, size_t lags, long long w0, long long w1,
-                                      long long chunk, double *sum, double *sq)
+__global__ void __launch_bounds__(FS_MOM_THREADS) fs_cor_moments_kernel(const unsigned char *cor, int lags, long long w0,
+                                                                        long long w1, double *part)
 {
     constexpr int NC = KIND == 2 ? 3 : 1;
-    const long long wb = w0 + (long long)blockIdx.x * chunk;
-    const long long we = wb + chunk < w1 ? wb + chunk : w1;
-    for (size_t l = threadIdx.x; l < lags; l += blockDim.x) {
+    __shared__ double red[2 * NC][FS_MOM_THREADS];
+    const int rows = lags < FS_MOM_THREADS ? FS_MOM_THREADS / lags : 1;  // walkers at a time
+    const int r = threadIdx.x / lags;
+    double *mine = part + (size_t)blockIdx.x * lags * 2 * NC;
+    for (int l0 = 0; l0 < lags; l0 += FS_MOM_THREADS) {
+        const int l = rows > 1 ? (int)threadIdx.x % lags : l0 + (int)threadIdx.x;
         double s[NC], q[NC];
 #pragma unroll
         for (int k = 0; k < NC; k++) s[k] = q[k] = 0.0;
-        for (long long w = wb; w < we; w++) {
-            const size_t i = (size_t)w * lags + l;
-            double v[NC];
-            if (KIND == 0) {
-                v[0] = (double)((const float *)cor)[i];
-            } else if (KIND == 1) {
-                v[0] = ((const double *)cor)[i];
-            } else {
-                const unsigned char *e = cor + i * 24;
-                v[0] = (double)*(const float *)(e + 8);
-                v[NC > 1 ? 1 : 0] = (double)*(const float *)(e + 12);
-                v[NC > 2 ? 2 : 0] = *(const double *)e;
+        if (l < lags && (rows == 1 || r < rows))
+            for (long long w = w0 + (long long)blockIdx.x * rows + (rows > 1 ? r : 0); w < w1;
+                 w += (long long)gridDim.x * rows) {
+                const size_t i = (size_t)w * lags + l;
+                double v[NC];
+                if (KIND == 0) {
+                    v[0] = (double)((const float *)cor)[i];
+                } else if (KIND == 1) {
+                    v[0] = ((const double *)cor)[i];
+                } else {
+                    const unsigned char *e = cor + i * 24;
+                    v[0] = (double)*(const float *)(e + 8);
+                    v[NC > 1 ? 1 : 0] = (double)*(const float *)(e + 12);
+                    v[NC > 2 ? 2 : 0] = *(const double *)e;
+                }
+#pragma unroll
+                for (int k = 0; k < NC; k++) {
+                    s[k] += v[k];
+                    q[k] += v[k] * v[k];
+                }
             }
+        if (rows > 1) {
 #pragma unroll
             for (int k = 0; k < NC; k++) {
-                s[k] += v[k];
-                q[k] += v[k] * v[k];
+                red[2 * k][threadIdx.x] = s[k];
+                red[2 * k + 1][threadIdx.x] = q[k];
             }
-        }
+            __syncthreads();
+            if (threadIdx.x < lags)
+                for (int j = 1; j < rows; j++)
 #pragma unroll
-        for (int k = 0; k < NC; k++) {
-            atomicAdd(sum + l * NC + k, s[k]);
-            atomicAdd(sq + l * NC + k, q[k]);
+                    for (int k = 0; k < NC; k++) {
+                        s[k] += red[2 * k][j * lags + l];
+                        q[k] += red[2 * k + 1][j * lags + l];
+                    }
         }
+        if (l < lags && (rows == 1 || r == 0))
+#pragma unroll
+            for (int k = 0; k < NC; k++) {
+                mine[(size_t)l * NC + k] = s[k];
+                mine[(size_t)(lags + l) * NC + k] = q[k];
+            }
+    }
+}
+
+__global__ void __launch_bounds__(FS_MOM_THREADS) fs_cor_moments_add_kernel(const double *part, int rows, int cols,
+                                                                            double *out)
+{
+    __shared__ double red[FS_MOM_THREADS / 32][32];
+    const int c = blockIdx.x * 32 + threadIdx.x % 32, g = threadIdx.x / 32;
+    double s = 0.0;
+    if (c < cols)
+        for (int r = g; r < rows; r += FS_MOM_THREADS / 32) s += part[(size_t)r * cols + c];
+    red[g][threadIdx.x % 32] = s;
+    __syncthreads();
+    if (g == 0 && c < cols) {
+#pragma unroll
+        for (int k = 1; k < FS_MOM_THREADS / 32; k++) s += red[k][threadIdx.x];
+        out[c] = s;
     }
 }
 
@@ -1640,27 +1752,26 @@ extern "C" int fs_reduce_correlator(fs_handle *h, int64_t walker_begin, int64_t 
         return fail(h, FS_ERR_IO, "walker range [%lld, %lld) outside [0, %zu)", (long long)walker_begin,
                     (long long)walker_end, W);
     CUDA_TRY(h, cudaSetDevice(h->device), FS_ERR_CUDA);
-    if (!h->d_red) CUDA_TRY(h, cudaMalloc((void **)&h->d_red, 2 * lags * 3 * sizeof(double)), FS_ERR_OOM);
-    CUDA_TRY(h, cudaMemsetAsync(h->d_red, 0, 2 * n * sizeof(double), h->stream), FS_ERR_CUDA);
-    const long long nw = walker_end - walker_begin;
-    int sms = 152;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-    const long long blocks = std::min<long long>(nw, (long long)sms * 8);
-    const long long chunk = (nw + blocks - 1) / blocks;
-    const unsigned grid = (unsigned)((nw + chunk - 1) / chunk);
+    // two blocks per SM, unless the walkers are fewer or the rows would take more than 64 MB
+    const long long nw = walker_end - walker_begin, rows = std::max<long long>(1, FS_MOM_THREADS / (long long)lags);
+    const size_t cols = 2 * n;
+    const long long room = std::max<long long>(1, (64ll << 20) / (long long)(cols * sizeof(double)));
+    const long long most = std::min(std::min<long long>(2ll * device_sms(), room), ((long long)W + rows - 1) / rows);
+    const unsigned grid = (unsigned)std::min(most, (nw + rows - 1) / rows);
+    if (!h->d_red) CUDA_TRY(h, cudaMalloc((void **)&h->d_red, (size_t)(most + 1) * cols * sizeof(double)), FS_ERR_OOM);
     const unsigned char *c = (const unsigned char *)h->d_cor;
-    double *s = h->d_red, *q = h->d_red + n;
+    double *part = h->d_red + cols, *dst = h->h_red ? h->h_red : h->d_red;
     if (h->cor_elem == 24)
-        fs_cor_moments_kernel<2><<<grid, 256, 0, h->stream>>>(c, lags, walker_begin, walker_end, chunk, s, q);
+        fs_cor_moments_kernel<2><<<grid, FS_MOM_THREADS, 0, h->stream>>>(c, (int)lags, walker_begin, walker_end, part);
     else if (h->cor_elem == 8)
-        fs_cor_moments_kernel<1><<<grid, 256, 0, h->stream>>>(c, lags, walker_begin, walker_end, chunk, s, q);
+        fs_cor_moments_kernel<1><<<grid, FS_MOM_THREADS, 0, h->stream>>>(c, (int)lags, walker_begin, walker_end, part);
     else
-        fs_cor_moments_kernel<0><<<grid, 256, 0, h->stream>>>(c, lags, walker_begin, walker_end, chunk, s, q);
+        fs_cor_moments_kernel<0><<<grid, FS_MOM_THREADS, 0, h->stream>>>(c, (int)lags, walker_begin, walker_end, part);
+    fs_cor_moments_add_kernel<<<(unsigned)((cols + 31) / 32), FS_MOM_THREADS, 0, h->stream>>>(part, (int)grid, (int)cols,
+                                                                                             dst);
     CUDA_TRY(h, cudaGetLastError(), FS_ERR_LAUNCH);
-    CUDA_TRY(h, cudaMemcpyAsync(sum, s, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaMemcpyAsync(sumsq, q, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream), FS_ERR_LAUNCH);
-    return FS_OK;
+    int rc = result_out(h, sum, dst, n, dst == h->h_red);
+    return rc ? rc : result_out(h, sumsq, dst + n, n, dst == h->h_red);
 }
 
 extern "C" int fs_set_paths_tiled(fs_handle *h, const void *host, size_t n_template)

@@ -46,8 +46,9 @@ struct FsBatchSys {
     fs_u32 *wseeds;          // [walkers][4]
     fs_u32 *rtab;            // RANLUX: [threads][28] (the reference's table layout)
     fs_u32 *gtab;            // RANLUX: [walkers][28]
-    fs_u32 *accepts;         // [threads]
+    fs_u32 *accepts;         // [threads] (small batches: page-locked host memory)
     double *op_sums;         // [walkers][nops], accumulated over launches
+    double *op_host;         // small batches: op_sums again, in page-locked host memory; else null
     int n_walkers, N, S, tpw, wpb, nops, type, n_tiles;
     int op_runs, msteps;
     int global;              // 1: the tile works on its walkers' rows of `paths` in place
@@ -313,7 +314,12 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
                 sd.paths[base + i] = FSB_AT(smem + wi * wstride, d, sl);
             }
         }
-        for (int i = tid; i < n_here * sd.nops; i += blockDim.x) sd.op_sums[(size_t)w0 * sd.nops + i] += s_op[i];
+        for (int i = tid; i < n_here * sd.nops; i += blockDim.x) {
+            const size_t k = (size_t)w0 * sd.nops + i;
+            const double sum = sd.op_sums[k] + s_op[i];
+            sd.op_sums[k] = sum;
+            if (sd.op_host) sd.op_host[k] = sum;
+        }
     }
     __syncthreads();  // the next tile reuses the shared-memory tile
 #undef FSB_IDX

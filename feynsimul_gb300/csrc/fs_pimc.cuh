@@ -668,11 +668,15 @@ __device__ __forceinline__ bool fs_vec_finite(const FsVec v)
 // Every path value passes through the launch's path-out copy (or, for global paths, the
 // owner's final check), so one compare per value per launch finds any walker whose
 // proposals or potential blew up; the host reads the word at fs_sync.
+// The word is in page-locked host memory, so it is stored to and not updated atomically: of
+// several such walkers any one may be the one recorded.
 #define FS_STATUS_NONFINITE 1
 __device__ __forceinline__ void fs_flag_nonfinite(int *status, int walker)
 {
-    atomicOr(status, FS_STATUS_NONFINITE);
-    atomicCAS(status + 1, 0, walker + 1);
+    volatile int *st = status;
+    if (st[0]) return;
+    st[1] = walker + 1;
+    st[0] = FS_STATUS_NONFINITE;
 }
 
 // Per-launch segment offsets (RANLUX, parallel-path mode): the walker's offset stream feeds
