@@ -892,6 +892,15 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         long long by_threads = 2048 / h->block;
         long long by_regs = 65536 / (64ll * h->block);
         long long by_grid = (h->grid + device_sms() - 1) / device_sms();
+        // Learned proposal: every warp reads the network's 73 KB of weights each step, which come
+        // from L1 only while the CTAs leave it that much of the SM's 256 KB.  Two trimer CTAs of
+        // 54 KB (132 KB carve-out) with twice the registers beat four that fetch the weights from
+        // L2: 8192 walkers, 10 sweeps, 1604 -> 1067 us (three CTAs: 1296).  Fewer than 8 warps
+        // per SM would not pay.
+        if (c.learned) {
+            const long long by_l1 = (132ll * 1024) / std::max<long long>(1, (long long)h->smem + 1024);
+            if (by_l1 * h->block >= 256) by_smem = std::min(by_smem, by_l1);
+        }
         h->cfg.min_blocks_per_sm =
             (int)std::max(1ll, std::min(std::min(std::min(by_smem, by_threads), by_regs), by_grid));
     }
