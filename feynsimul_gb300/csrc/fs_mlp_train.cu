@@ -49,8 +49,14 @@ __device__ __forceinline__ fs_bf16 f2bf(float x)
 
 // ---------------------------------------------------------------- tcgen05 training
 // The same forward pass, loss and backward pass on the fifth-generation tensor cores, with
-// the same BF16 rounding points.  One CTA = 4 warps, persistent over 128-row tiles; thread t
-// owns row t of a tile (tensor-memory lane t) in every epilogue.  Tensor memory (512 FP32
+// the same BF16 rounding points.  One CTA = 8 warps, persistent over 128-row tiles; a row of a
+// tile (a tensor-memory lane) belongs to two threads, r and r + 128, which take half of its
+// columns each in every epilogue (a warp reads the 32 lanes of its number modulo 4).  The step is
+// a chain of 8 MMA groups with an epilogue between; of one tile's 34 thousand cycles (42 with one
+// warp a lane quarter and gradients stored line by line) the MMAs and their waits are about 7, the
+// epilogues 15, the weights 5 and the gradient's way out 5.  A step on 4096 rows, optimiser and
+// gather included, took 105 us in ten launches and takes 31 in three.
+// Rows of a training set are gathered in place by an index array.  Tensor memory (512 FP32
 // columns): the layer accumulator F (a forward layer's output or a hidden gradient dA), and
 // the weight gradients summed over the CTA's tiles: dW2 and dW3 (128 columns each), dW1 (16)
 // and dW4 transposed (16; its M is the 128 inputs).  Shared memory holds BF16 tiles in the
@@ -60,9 +66,12 @@ __device__ __forceinline__ fs_bf16 f2bf(float x)
 // MN-major, and dW = dZ^T A reads dZ and A MN-major (K = the tile's rows), so no tile is
 // transposed.  The six 128-wide tiles come first and the allocation is padded, so every
 // byte a descriptor can reach lies inside it under either reading of its byte offsets.
-// Bias gradients are FP32 column sums of the unrounded gradients (warp butterflies, then
-// shared-memory atomics).
-#define TT_THREADS 128
+// Bias gradients are FP32 column sums of the unrounded gradients (warp butterflies, each quarter
+// of the rows on its own, then the quarters in order).
+// A CTA's gradient goes to its own row of `part` for the optimiser step to add up in order
+// (fs_mlp_train_batch: the same training run gives the same bits), or, without one, to grad
+// by atomics (fs_mlp_train_step).
+#define TT_THREADS 256
 #define TT_TMEM_COLS 512
 #define TT_F 0u
 #define TT_DW2 128u
@@ -82,8 +91,8 @@ struct TtSmem {
     alignas(128) fs_bf16 dz4[128 * 16];
     alignas(128) fs_bf16 w1[128 * 16];
     float bias[128 * 3 + 16];
-    float db[128 * 3 + 16];
-    float loss;
+    float db[4][128 * 3 + 16];  // bias gradients of each quarter of a tile's rows
+    float loss[4];
     alignas(8) unsigned long long mbar;
     unsigned tmem_base;
     int give_up;
@@ -94,8 +103,15 @@ struct TtSmem {
 #define TT_SMEM_BYTES \
     (offsetof(TtSmem, g) + TT_REACH > sizeof(TtSmem) ? offsetof(TtSmem, g) + TT_REACH : sizeof(TtSmem))
 
+// A row of `part`: a gradient in the parameters' order, but W1..W3 by quads of inputs, (input / 4,
+// output, input mod 4), so that a warp of tensor-memory lanes (outputs) writes 512 consecutive bytes
+// (in the parameters' order each of its 16-byte stores is a line of its own, and the 144 KB took 12
+// of the pass's 42 thousand cycles); then the loss, padded to 16 floats
+__device__ __forceinline__ int tt_quad(int row, int col, int rows) { return (col >> 2) * 4 * rows + row * 4 + (col & 3); }
+#define TT_PART ((FS_MLP_NPARAM + 1 + 15) / 16 * 16)
+
 // column sums over the warp's 32 lanes of v[0..32) (one value per column and lane), added to
-// dst[lane] for lane < ncols; v is consumed
+// dst[lane] for lane < ncols (no other warp adds there); v is consumed
 __device__ __forceinline__ void tt_colsum32(float (&v)[32], float *dst, int lane, int ncols)
 {
 #pragma unroll
@@ -108,42 +124,64 @@ __device__ __forceinline__ void tt_colsum32(float (&v)[32], float *dst, int lane
             v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, w);
         }
     }
-    if (lane < ncols) atomicAdd(dst + lane, v[0]);
+    if (lane < ncols) dst[lane] += v[0];
 }
 
 __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
     const float *__restrict__ params, const fs_bf16 *__restrict__ wq, float *__restrict__ grad,
-    const float *__restrict__ xin, const float *__restrict__ zin, int n_rows, int dof, float inv_batch,
-    float *loss_out)
+    const float *__restrict__ xin, const float *__restrict__ zin, const long long *__restrict__ pick, int n_rows,
+    int dof, float inv_batch, float *loss_out, float *part)
 {
     extern __shared__ __align__(1024) unsigned char tt_raw[];
     TtSmem &S = *reinterpret_cast<TtSmem *>(tt_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int r = tid & 127, half = tid >> 7;  // row of the tile, half of its columns
     const int n_tiles = (n_rows + 127) / 128;
     const uint32_t mbar = tc_smem(&S.mbar);
 
+    // ---- the first tile's rows, ahead of the weights ----
+    const int row0 = (int)blockIdx.x * 128 + r;
+    const bool valid0 = row0 < n_rows;
+    size_t src = valid0 && pick ? (size_t)pick[row0] : (size_t)row0;
+    // half a row of x, and the row's z (the threads of half 0 use it)
+    float4 xv[2], zv[2];
+    auto fetch = [&](bool valid) {
+        const float4 *xr = reinterpret_cast<const float4 *>(xin + src * 16 + 8 * half);
+#pragma unroll
+        for (int c = 0; c < 2; c++) xv[c] = valid ? xr[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+        float *z = reinterpret_cast<float *>(zv);
+#pragma unroll
+        for (int d = 0; d < 8; d++) z[d] = valid && half == 0 && d < dof ? zin[src * 8 + d] : 0.f;
+    };
     // ---- weights (the BF16 training copy, [out][in]) into canonical tiles, eight
-    // consecutive inputs (one core-matrix row, 16 bytes) per load and store; biases ----
+    // consecutive inputs (one core-matrix row, 16 bytes) per load and store; a warp takes 8
+    // rows of 4 core matrices: 64 contiguous bytes of each row, 512 of the tile ----
     {
         const uint4 *q = reinterpret_cast<const uint4 *>(wq);
-        for (int i = tid; i < 128 * 16 / 8; i += TT_THREADS)
-            *reinterpret_cast<uint4 *>(S.w1 + tc_off(i / 2, (i % 2) * 8, 16)) = q[Q_W1 / 8 + i];
-        for (int i = tid; i < 128 * 128 / 8; i += TT_THREADS) {
-            *reinterpret_cast<uint4 *>(S.w2 + tc_off(i / 16, (i % 16) * 8, 128)) = q[Q_W2 / 8 + i];
-            *reinterpret_cast<uint4 *>(S.w3 + tc_off(i / 16, (i % 16) * 8, 128)) = q[Q_W3 / 8 + i];
-        }
-        for (int i = tid; i < 16 * 128 / 8; i += TT_THREADS)
-            *reinterpret_cast<uint4 *>(S.w4 + tc_off(i / 16, (i % 16) * 8, 128)) = q[Q_W4 / 8 + i];
+        const int lr = lane & 7, lk = lane >> 3;
+        auto tile128 = [&](fs_bf16 *w, int off, int rows) {
+#pragma unroll 8
+            for (int i = warp; i < rows / 8 * 4; i += TT_THREADS / 32) {
+                const int row = i / 4 * 8 + lr, k = i % 4 * 4 + lk;
+                *reinterpret_cast<uint4 *>(w + tc_off(row, k * 8, 128)) = q[off / 8 + row * 16 + k];
+            }
+        };
+        tile128(S.w2, Q_W2, 128);
+        tile128(S.w3, Q_W3, 128);
+        tile128(S.w4, Q_W4, 16);
+        const int row = warp * 16 + (lane & 15), k = lane >> 4;  // 8 warps x 16 rows of 2 core matrices
+        *reinterpret_cast<uint4 *>(S.w1 + tc_off(row, k * 8, 16)) = q[Q_W1 / 8 + row * 2 + k];
     }
+    fetch(valid0);
     for (int i = tid; i < 128; i += TT_THREADS) {
         S.bias[i] = params[P_B1 + i];
         S.bias[128 + i] = params[P_B2 + i];
         S.bias[256 + i] = params[P_B3 + i];
     }
     if (tid < 16) S.bias[384 + tid] = params[P_B4 + tid];
-    for (int i = tid; i < 128 * 3 + 16; i += TT_THREADS) S.db[i] = 0.f;
+    for (int i = tid; i < 4 * (128 * 3 + 16); i += TT_THREADS) S.db[0][i] = 0.f;
+    if (tid < 4) S.loss[tid] = 0.f;
     if (tid == 0) {
-        S.loss = 0.f;
         S.give_up = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -159,9 +197,10 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = S.tmem_base;
-    const uint32_t t_row = tmem + ((uint32_t)(32 * warp) << 16);  // this warp's lanes
+    const uint32_t t_row = tmem + ((uint32_t)(32 * (warp & 3)) << 16);  // this warp's lanes
     uint32_t phase = 0;
     bool ok = true, first = true;
+    float *const db = S.db[warp & 3];
 
     // one step: the operands made visible to the tensor cores, thread 0 issues the MMAs and
     // commits, every thread waits (bounded) for them
@@ -184,54 +223,45 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
     // forward epilogue: act = BF16(relu(F + b))
     auto relu_out = [&](fs_bf16 *act, const float *b) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 16) {
+        for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 16) {
             float v[16];
             tc_ld16(t_row + TT_F + (uint32_t)c0, v);
 #pragma unroll
             for (int i = 0; i < 16; i++) v[i] = fmaxf(v[i] + b[c0 + i], 0.f);
-            tc_st8(act + tc_off(tid, c0, 128), v);
-            tc_st8(act + tc_off(tid, c0 + 8, 128), v + 8);
+            tc_st8(act + tc_off(r, c0, 128), v);
+            tc_st8(act + tc_off(r, c0 + 8, 128), v + 8);
         }
     };
     // backward epilogue: dZ = F * (act > 0) -> g as BF16, its FP32 column sums into dbl
     auto grad_out = [&](const fs_bf16 *act, float *dbl) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 32) {
+        for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 32) {
             float v[32];
             tc_ld16(t_row + TT_F + (uint32_t)c0, *reinterpret_cast<float(*)[16]>(v));
             tc_ld16(t_row + TT_F + (uint32_t)c0 + 16u, *reinterpret_cast<float(*)[16]>(v + 16));
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const uint4 u = *reinterpret_cast<const uint4 *>(act + tc_off(tid, c0 + 8 * q, 128));
+                const uint4 u = *reinterpret_cast<const uint4 *>(act + tc_off(r, c0 + 8 * q, 128));
                 const unsigned w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     if (!(__uint_as_float(w[e] << 16) > 0.f)) v[8 * q + 2 * e] = 0.f;
                     if (!(__uint_as_float(w[e] & 0xFFFF0000u) > 0.f)) v[8 * q + 2 * e + 1] = 0.f;
                 }
-                tc_st8(S.g + tc_off(tid, c0 + 8 * q, 128), v + 8 * q);
+                tc_st8(S.g + tc_off(r, c0 + 8 * q, 128), v + 8 * q);
             }
             tt_colsum32(v, dbl + c0, lane, 32);
         }
     };
 
     for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const int row = tile * 128 + tid;
+        const int row = tile * 128 + r;
         const bool valid = row < n_rows;
-        {
-            float h[16];
-            const float4 *xr = reinterpret_cast<const float4 *>(xin + (size_t)row * 16);
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const float4 f = valid ? xr[c] : make_float4(0.f, 0.f, 0.f, 0.f);
-                h[4 * c] = f.x;
-                h[4 * c + 1] = f.y;
-                h[4 * c + 2] = f.z;
-                h[4 * c + 3] = f.w;
-            }
-            tc_st8(S.x + tc_off(tid, 0, 16), h);
-            tc_st8(S.x + tc_off(tid, 8, 16), h + 8);
+        if (tile != (int)blockIdx.x) {
+            src = valid && pick ? (size_t)pick[row] : (size_t)row;
+            fetch(valid);
         }
+        tc_st8(S.x + tc_off(r, 8 * half, 16), reinterpret_cast<const float *>(xv));
         // ---- forward ----
         if (!step([&] { tc_mma(tmem + TT_F, tc_desc(S.x, 16), tc_desc(S.w1, 16), tc_idesc(128, 128), 0); }))
             break;
@@ -257,7 +287,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
             }))
             break;
         // ---- loss and its gradient for this thread's row ----
-        {
+        if (half == 0) {
             float z4[16], g[32];
             tc_ld16(t_row + TT_F, z4);
 #pragma unroll
@@ -276,7 +306,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
                     const float th = tanhf(0.25f * sr);
                     const float s = 4.f * th;
                     const float e = expf(-s);
-                    const float z = zin[(size_t)row * 8 + d];
+                    const float z = reinterpret_cast<const float *>(zv)[d];
                     const float df = z - o;
                     l += 0.5f * df * df * e + 0.5f * s;
                     g[d] = -df * e * inv_batch;
@@ -285,12 +315,12 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
                     for (int c = 0; c < 16; c++) g[c] = c == dof + d ? gs : g[c];
                 }
             }
-            tc_st8(S.dz4 + tc_off(tid, 0, 16), g);
-            tc_st8(S.dz4 + tc_off(tid, 8, 16), g + 8);
+            tc_st8(S.dz4 + tc_off(r, 0, 16), g);
+            tc_st8(S.dz4 + tc_off(r, 8, 16), g + 8);
 #pragma unroll
             for (int off = 16; off >= 1; off >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, off);
-            if (lane == 0) atomicAdd(&S.loss, l);
-            tt_colsum32(g, S.db + 384, lane, 16);
+            if (lane == 0) S.loss[warp] += l;
+            tt_colsum32(g, db + 384, lane, 16);
         }
         // ---- backward ----
         const uint32_t acc0 = first ? 0u : 1u;
@@ -302,7 +332,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
                 tc_mma(tmem + TT_F, tc_desc(S.dz4, 16), tc_desc_mn(S.w4, 128), tc_idesc(128, 128, false, true), 0);
             }))
             break;
-        grad_out(S.a3, S.db + 256);
+        grad_out(S.a3, db + 256);
         if (!step([&] {
                 for (int kk = 0; kk < 8; kk++)  // dW3 += dZ3^T A2
                     tc_mma(tmem + TT_DW3, tc_desc_mn(S.g + kk * 2048, 128), tc_desc_mn(S.a2 + kk * 2048, 128),
@@ -312,7 +342,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
                            tc_idesc(128, 128, false, true), kk > 0);
             }))
             break;
-        grad_out(S.a2, S.db + 128);
+        grad_out(S.a2, db + 128);
         if (!step([&] {
                 for (int kk = 0; kk < 8; kk++)  // dW2 += dZ2^T A1
                     tc_mma(tmem + TT_DW2, tc_desc_mn(S.g + kk * 2048, 128), tc_desc_mn(S.a1 + kk * 2048, 128),
@@ -322,7 +352,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
                            tc_idesc(128, 128, false, true), kk > 0);
             }))
             break;
-        grad_out(S.a1, S.db);
+        grad_out(S.a1, db);
         if (!step([&] {
                 for (int kk = 0; kk < 8; kk++)  // dW1 += dZ1^T X
                     tc_mma(tmem + TT_DW1, tc_desc_mn(S.g + kk * 2048, 128), tc_desc_mn(S.x + kk * 256, 16),
@@ -332,40 +362,52 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
         first = false;
     }
     if (ok && !first) {
-        // the CTA's weight gradients out of tensor memory: thread t = lane t is output row t
-        // of dW1..dW3 and input column t of dW4
+        // the CTA's weight gradients out of tensor memory: lane r is output row r of dW1..dW3 and
+        // input column r of dW4; the row's two threads take dW2, dW1 and dW3, dW4
         // (16-byte vector atomics: the parameter offsets of W1..W3 are multiples of 4 floats)
-        auto add4 = [](float *dst, const float *v) {
-            atomicAdd(reinterpret_cast<float4 *>(dst), make_float4(v[0], v[1], v[2], v[3]));
+        float *const out = part ? part + (size_t)blockIdx.x * TT_PART : grad;
+        auto put4 = [&](float *dst, const float *v) {
+            const float4 f = make_float4(v[0], v[1], v[2], v[3]);
+            if (part) *reinterpret_cast<float4 *>(dst) = f;
+            else atomicAdd(reinterpret_cast<float4 *>(dst), f);
         };
-#pragma unroll 1
+        auto put = [&](float *dst, float v) {
+            if (part) *dst = v;
+            else atomicAdd(dst, v);
+        };
+        const uint32_t t_dw = t_row + (half == 0 ? TT_DW2 : TT_DW3);
+        const int p_w = half == 0 ? P_W2 : P_W3;
+#pragma unroll 2
         for (int c0 = 0; c0 < 128; c0 += 16) {
             float v[16];
-            tc_ld16(t_row + TT_DW2 + (uint32_t)c0, v);
+            tc_ld16(t_dw + (uint32_t)c0, v);
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) add4(grad + P_W2 + tid * 128 + c0 + i, v + i);
-            tc_ld16(t_row + TT_DW3 + (uint32_t)c0, v);
-#pragma unroll
-            for (int i = 0; i < 16; i += 4) add4(grad + P_W3 + tid * 128 + c0 + i, v + i);
+            for (int i = 0; i < 16; i += 4) put4(out + p_w + (part ? tt_quad(r, c0 + i, 128) : r * 128 + c0 + i), v + i);
         }
         {
             float v[16];
-            tc_ld16(t_row + TT_DW1, v);
+            tc_ld16(t_row + (half == 0 ? TT_DW1 : TT_DW4), v);
+            if (half == 0) {
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) add4(grad + P_W1 + tid * 16 + i, v + i);
-            tc_ld16(t_row + TT_DW4, v);
+                for (int i = 0; i < 16; i += 4) put4(out + P_W1 + (part ? tt_quad(r, i, 128) : r * 16 + i), v + i);
+            } else {
 #pragma unroll
-            for (int o = 0; o < 16; o++) atomicAdd(grad + P_W4 + o * 128 + tid, v[o]);
+                for (int o = 0; o < 16; o++) put(out + P_W4 + o * 128 + r, v[o]);
+            }
         }
-        for (int i = tid; i < 128; i += TT_THREADS) {
-            atomicAdd(grad + P_B1 + i, S.db[i]);
-            atomicAdd(grad + P_B2 + i, S.db[128 + i]);
-            atomicAdd(grad + P_B3 + i, S.db[256 + i]);
+        auto quarters = [&](int i) { return (S.db[0][i] + S.db[1][i]) + (S.db[2][i] + S.db[3][i]); };
+        if (tid < 128) {
+            put(out + P_B1 + tid, quarters(tid));
+            put(out + P_B2 + tid, quarters(128 + tid));
+            put(out + P_B3 + tid, quarters(256 + tid));
         }
-        if (tid < 16) atomicAdd(grad + P_B4 + tid, S.db[384 + tid]);
-        if (tid == 0 && loss_out) atomicAdd(loss_out, S.loss);
+        if (tid < 16) put(out + P_B4 + tid, quarters(384 + tid));
+        const float loss = (S.loss[0] + S.loss[1]) + (S.loss[2] + S.loss[3]);
+        if (tid == 0 && part) out[FS_MLP_NPARAM] = loss;
+        if (tid == 0 && !part && loss_out) atomicAdd(loss_out, loss);
     }
-    if (!ok && tid == 0 && loss_out) atomicAdd(loss_out, __int_as_float(0x7FC00000));  // gave up: NaN loss
+    if (!ok && tid == 0 && part) part[(size_t)blockIdx.x * TT_PART + FS_MLP_NPARAM] = __int_as_float(0x7FC00000);
+    if (!ok && tid == 0 && !part && loss_out) atomicAdd(loss_out, __int_as_float(0x7FC00000));  // gave up: NaN loss
     // release the tensor memory once no MMA is in flight: after a give-up, wait (bounded)
     // for the last commit's phase before freeing the columns
     if (!ok) tc_wait(mbar, phase ^ 1u);
@@ -377,28 +419,62 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
                      : "memory");
 }
 
-// Adam step on the FP32 master weights; writes the BF16 training copy and clears the
-// gradient.
-__global__ void fs_mlp_adam_kernel(float *params, float *m, float *v, float *grad, fs_bf16 *wq, float lr,
-                                   float b1c, float b2c)
+// one parameter's Adam step on the FP32 master weights; writes the BF16 training copy
+__device__ __forceinline__ void adam_one(int i, float g, float w0, float m0, float v0, float *params, float *m,
+                                         float *v, fs_bf16 *wq, float lr, float b1c, float b2c)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= FS_MLP_NPARAM) return;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const float g = grad[i];
-    const float mi = b1 * m[i] + (1.f - b1) * g;
-    const float vi = b2 * v[i] + (1.f - b2) * g * g;
+    const float mi = b1 * m0 + (1.f - b1) * g;
+    const float vi = b2 * v0 + (1.f - b2) * g * g;
     m[i] = mi;
     v[i] = vi;
-    const float w = params[i] - lr * (mi / b1c) / (sqrtf(vi / b2c) + eps);
+    const float w = w0 - lr * (mi / b1c) / (sqrtf(vi / b2c) + eps);
     params[i] = w;
-    grad[i] = 0.f;
     int q = -1;
     if (i < P_B1) q = Q_W1 + (i - P_W1);
     else if (i >= P_W2 && i < P_B2) q = Q_W2 + (i - P_W2);
     else if (i >= P_W3 && i < P_B3) q = Q_W3 + (i - P_W3);
     else if (i >= P_W4 && i < P_B4) q = Q_W4 + (i - P_W4);
     if (q >= 0) wq[q] = f2bf(w);
+}
+
+// Adam step; clears the gradient.
+__global__ void fs_mlp_adam_kernel(float *params, float *m, float *v, float *grad, fs_bf16 *wq, float lr,
+                                   float b1c, float b2c)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= FS_MLP_NPARAM) return;
+    adam_one(i, grad[i], params[i], m[i], v[i], params, m, v, wq, lr, b1c, b2c);
+    grad[i] = 0.f;
+}
+
+// Adam step on the gradient that n_parts CTAs of the training pass left in their rows of part:
+// added in order with the rounding errors on the side (TwoSum), so the sum is the exact one
+// rounded once or twice, and the same whenever the rows are.  The last thread adds the losses.
+__global__ void fs_mlp_adam_parts_kernel(const float *__restrict__ part, int n_parts, float *params, float *m, float *v,
+                                         fs_bf16 *wq, float lr, float b1c, float b2c, float *loss_out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > FS_MLP_NPARAM) return;
+    // the parameter at place i of the row (tt_quad)
+    int p = i;
+    if (i < P_B1) p = P_W1 + (i - P_W1) % 512 / 4 * 16 + (i - P_W1) / 512 * 4 + i % 4;
+    else if (i >= P_W2 && i < P_B2) p = P_W2 + (i - P_W2) % 512 / 4 * 128 + (i - P_W2) / 512 * 4 + i % 4;
+    else if (i >= P_W3 && i < P_B3) p = P_W3 + (i - P_W3) % 512 / 4 * 128 + (i - P_W3) / 512 * 4 + i % 4;
+    const bool param = i < FS_MLP_NPARAM;
+    const float w0 = param ? params[p] : 0.f, m0 = param ? m[p] : 0.f, v0 = param ? v[p] : 0.f;
+    float s = 0.f, e = 0.f;
+#pragma unroll 16
+    for (int k = 0; k < n_parts; k++) {
+        const float x = part[(size_t)k * TT_PART + i];
+        const float t = __fadd_rn(s, x);
+        const float bp = __fsub_rn(t, s);
+        e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, bp)), __fsub_rn(x, bp)));
+        s = t;
+    }
+    const float g = __fadd_rn(s, e);
+    if (param) adam_one(p, g, w0, m0, v0, params, m, v, wq, lr, b1c, b2c);
+    else if (loss_out) *loss_out = g;
 }
 
 // FP32 master weights -> BF16 training copy + inference fragments + biases
@@ -457,6 +533,29 @@ extern "C" int fs_mlp_sizes(int64_t *n_param, int64_t *n_bf16, int64_t *n_frag_u
     return FS_OK;
 }
 
+// CTAs of a pass over n_rows: one per 128-row tile, at most one per SM
+static int train_ctas(int n_rows)
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int n_tiles = (n_rows + 127) / 128;
+    return n_tiles < sms ? n_tiles : sms < 1 ? 1 : sms;
+}
+
+static int train_pass(const float *params, const uint16_t *wq, float *grad, const float *x, const float *z,
+                      const long long *pick, int32_t n_rows, int32_t dof, float inv_batch, float *loss, float *part,
+                      int ctas, void *stream)
+{
+    // per call: the attribute belongs to the current device (a process may use several)
+    cudaError_t e = cudaFuncSetAttribute(fs_mlp_train_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)TT_SMEM_BYTES);
+    if (e != cudaSuccess) return fsi_thread_error(FS_ERR_CUDA, cudaGetErrorString(e));
+    fs_mlp_train_tc_kernel<<<ctas, TT_THREADS, TT_SMEM_BYTES, (cudaStream_t)stream>>>(
+        params, (const fs_bf16 *)wq, grad, x, z, pick, n_rows, dof, inv_batch, loss, part);
+    return launch_check("fs_mlp_train_tc_kernel");
+}
+
 extern "C" int fs_mlp_train_step(const float *params, const uint16_t *wq, float *grad, const float *x,
                                  const float *z, int32_t n_rows, int32_t dof, float inv_batch, float *loss,
                                  void *stream)
@@ -465,18 +564,7 @@ extern "C" int fs_mlp_train_step(const float *params, const uint16_t *wq, float 
         return fsi_thread_error(FS_ERR_CONFIG, "fs_mlp_train_step: need 1 <= dof <= 8 and n_rows >= 1");
     if (((uintptr_t)wq | (uintptr_t)x | (uintptr_t)grad) & 15u)
         return fsi_thread_error(FS_ERR_CONFIG, "fs_mlp_train_step: wq, x and grad must be 16-byte aligned");
-    // per call: the attribute belongs to the current device (a process may use several)
-    cudaError_t e = cudaFuncSetAttribute(fs_mlp_train_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)TT_SMEM_BYTES);
-    if (e != cudaSuccess) return fsi_thread_error(FS_ERR_CUDA, cudaGetErrorString(e));
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms < 1) sms = 1;
-    const int n_tiles = (n_rows + 127) / 128;
-    fs_mlp_train_tc_kernel<<<n_tiles < sms ? n_tiles : sms, TT_THREADS, TT_SMEM_BYTES, (cudaStream_t)stream>>>(
-        params, (const fs_bf16 *)wq, grad, x, z, n_rows, dof, inv_batch, loss);
-    return launch_check("fs_mlp_train_tc_kernel");
+    return train_pass(params, wq, grad, x, z, nullptr, n_rows, dof, inv_batch, loss, nullptr, train_ctas(n_rows), stream);
 }
 
 extern "C" int fs_mlp_adam(float *params, float *m, float *v, float *grad, uint16_t *wq, int32_t step, float lr,
@@ -487,6 +575,35 @@ extern "C" int fs_mlp_adam(float *params, float *m, float *v, float *grad, uint1
     fs_mlp_adam_kernel<<<(FS_MLP_NPARAM + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
         params, m, v, grad, (fs_bf16 *)wq, lr, b1c, b2c);
     return launch_check("fs_mlp_adam_kernel");
+}
+
+extern "C" int fs_mlp_workspace(int32_t n_rows, int64_t *n_floats)
+{
+    if (n_rows < 1 || !n_floats) return fsi_thread_error(FS_ERR_CONFIG, "fs_mlp_workspace: need n_rows >= 1");
+    *n_floats = (int64_t)train_ctas(n_rows) * TT_PART;
+    return FS_OK;
+}
+
+extern "C" int fs_mlp_train_batch(float *params, float *m, float *v, uint16_t *wq, const float *x, const float *z,
+                                  const int64_t *rows, int32_t n_rows, int32_t dof, float *loss, int32_t step,
+                                  float lr, float *workspace, int64_t n_workspace, void *stream)
+{
+    if (dof < 1 || dof > 8 || n_rows < 1 || step < 1 || !rows || !workspace)
+        return fsi_thread_error(FS_ERR_CONFIG,
+                                "fs_mlp_train_batch: need rows, a workspace, 1 <= dof <= 8, n_rows >= 1 and step >= 1");
+    if (((uintptr_t)wq | (uintptr_t)x | (uintptr_t)workspace) & 15u)
+        return fsi_thread_error(FS_ERR_CONFIG, "fs_mlp_train_batch: wq, x and workspace must be 16-byte aligned");
+    const int ctas = train_ctas(n_rows);
+    if (n_workspace < (int64_t)ctas * TT_PART)
+        return fsi_thread_error(FS_ERR_CONFIG, "fs_mlp_train_batch: workspace smaller than fs_mlp_workspace asks for");
+    static_assert(sizeof(long long) == sizeof(int64_t), "row numbers");
+    int rc = train_pass(params, wq, nullptr, x, z, (const long long *)rows, n_rows, dof, (float)(1.0 / n_rows), nullptr,
+                        workspace, ctas, stream);
+    if (rc) return rc;
+    const float b1c = 1.f - powf(0.9f, (float)step), b2c = 1.f - powf(0.999f, (float)step);
+    fs_mlp_adam_parts_kernel<<<FS_MLP_NPARAM / 128 + 1, 128, 0, (cudaStream_t)stream>>>(
+        workspace, ctas, params, m, v, (fs_bf16 *)wq, lr, b1c, b2c, loss);
+    return launch_check("fs_mlp_adam_parts_kernel");
 }
 
 extern "C" int fs_mlp_pack(const float *params, uint16_t *wq, void *frag, float *bias, void *stream)

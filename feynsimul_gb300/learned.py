@@ -161,13 +161,20 @@ class LearnedProposal:
         """Raw network outputs (n, 16) for features (n, 16), via fs_mlp_infer."""
         import torch
         L = _lib.lib()
-        frag, bias = self.packed()
         dev = "cuda"
-        tf = torch.from_numpy(frag.view(np.uint8).copy()).to(dev)
-        tb = torch.from_numpy(bias).to(dev)
+        s = torch.cuda.current_stream().cuda_stream
+        sizes = [ctypes.c_int64() for _ in range(4)]
+        _lib.check(L.fs_mlp_sizes(*[ctypes.byref(v) for v in sizes]))
+        params = np.ascontiguousarray(self.params, np.float32).ravel()
+        if params.size < sizes[0].value:
+            raise ValueError(f"the network has {sizes[0].value} parameters, got {params.size}")
+        tp = torch.from_numpy(params).to(dev)
+        tq = torch.empty(sizes[1].value, dtype=torch.int16, device=dev)
+        tf = torch.empty(sizes[2].value * 2, dtype=torch.int32, device=dev)
+        tb = torch.empty(sizes[3].value, dtype=torch.float32, device=dev)
+        _lib.check(L.fs_mlp_pack(tp.data_ptr(), tq.data_ptr(), tf.data_ptr(), tb.data_ptr(), s))
         tx = torch.from_numpy(np.ascontiguousarray(feats, np.float32)).to(dev)
         ty = torch.zeros((tx.shape[0], OUT), dtype=torch.float32, device=dev)
-        s = torch.cuda.current_stream().cuda_stream
         _lib.check(L.fs_mlp_infer(tf.data_ptr(), tb.data_ptr(), tx.data_ptr(), ty.data_ptr(), tx.shape[0], s))
         torch.cuda.synchronize()
         return ty.cpu().numpy()
@@ -205,30 +212,29 @@ class LearnedProposal:
         tp = torch.from_numpy(self.params.copy()).to(dev)
         tm = torch.zeros_like(tp)
         tv = torch.zeros_like(tp)
-        tg = torch.zeros_like(tp)
+        need = ctypes.c_int64()
+        _lib.check(L.fs_mlp_workspace(batch, ctypes.byref(need)))
+        work = torch.empty(need.value, dtype=torch.float32, device=dev)
         tq = torch.zeros(n_bf16, dtype=torch.int16, device=dev)
         frag_dummy = torch.zeros(sizes[2].value * 2, dtype=torch.int32, device=dev)
         bias_dummy = torch.zeros(sizes[3].value, dtype=torch.float32, device=dev)
         tx = torch.from_numpy(np.ascontiguousarray(feats, np.float32)).to(dev)
         tz = torch.from_numpy(np.ascontiguousarray(targets, np.float32)).to(dev)
-        loss = torch.zeros(1, dtype=torch.float32, device=dev)
         stream = torch.cuda.current_stream().cuda_stream
         _lib.check(L.fs_mlp_pack(tp.data_ptr(), tq.data_ptr(), frag_dummy.data_ptr(), bias_dummy.data_ptr(), stream))
         gen = torch.Generator(device=dev)
         gen.manual_seed(seed)
-        losses = torch.zeros(steps, dtype=torch.float32, device=dev)
+        sums = torch.zeros(steps, dtype=torch.float32, device=dev)  # each step's loss over its batch
+        before_rows = tp.data_ptr(), tm.data_ptr(), tv.data_ptr(), tq.data_ptr(), tx.data_ptr(), tz.data_ptr()
+        sum_ptr, work_ptr = sums.data_ptr(), work.data_ptr()
         for it in range(steps):
+            # the training kernel gathers the batch's rows itself
             idx = torch.randint(0, n, (batch,), device=dev, generator=gen)
-            xb = tx.index_select(0, idx).contiguous()
-            zb = tz.index_select(0, idx).contiguous()
-            loss.zero_()
-            _lib.check(L.fs_mlp_train_step(tp.data_ptr(), tq.data_ptr(), tg.data_ptr(), xb.data_ptr(),
-                                           zb.data_ptr(), batch, self.dof, 1.0 / batch, loss.data_ptr(), stream))
-            _lib.check(L.fs_mlp_adam(tp.data_ptr(), tm.data_ptr(), tv.data_ptr(), tg.data_ptr(), tq.data_ptr(),
-                                     it + 1, lr, stream))
-            losses[it] = loss[0] / batch
+            _lib.check(L.fs_mlp_train_batch(*before_rows, idx.data_ptr(), batch, self.dof, sum_ptr + 4 * it, it + 1, lr,
+                                            work_ptr, need.value, stream))
             if log_every and (it + 1) % log_every == 0:
-                print(f"step {it + 1}: loss {float(losses[it]):.4f}")
+                print(f"step {it + 1}: loss {float(sums[it] / batch):.4f}")
+        losses = sums / batch
         torch.cuda.synchronize()
         self.params = tp.cpu().numpy().astype(np.float32)
         hist = losses.cpu().numpy()

@@ -315,6 +315,15 @@ int fs_mlp_train_step(const float *params, const uint16_t *wq, float *grad, cons
 /* Adam (beta 0.9 / 0.999) on params; refreshes the BF16 copy wq; clears grad. */
 int fs_mlp_adam(float *params, float *m, float *v, float *grad, uint16_t *wq, int32_t step,
                 float lr, void *stream);
+/* One optimisation step on the rows of a training set that `rows` (device, n_rows numbers, each
+ * within the set) picks: the pass of fs_mlp_train_step over them with inv_batch = 1 / n_rows,
+ * gathered in place, and the Adam step of fs_mlp_adam; *loss becomes the batch's loss sum.  The
+ * CTAs' gradients pass through `workspace` (device, 16-byte aligned, fs_mlp_workspace floats) and
+ * are added in order, so equal runs give equal bits. */
+int fs_mlp_workspace(int32_t n_rows, int64_t *n_floats);
+int fs_mlp_train_batch(float *params, float *m, float *v, uint16_t *wq, const float *x, const float *z,
+                       const int64_t *rows, int32_t n_rows, int32_t dof, float *loss, int32_t step,
+                       float lr, float *workspace, int64_t n_workspace, void *stream);
 /* params -> BF16 training copy, inference fragments (n_frag_u2 x 8 bytes), biases. */
 int fs_mlp_pack(const float *params, uint16_t *wq, void *frag, float *bias, void *stream);
 /* Inference of rows x[n][16] -> y[n][16] on the tcgen05 tensor cores (BF16 operands in
