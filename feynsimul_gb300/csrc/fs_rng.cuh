@@ -528,6 +528,13 @@ struct FsRanluxStream {
     }
 };
 
+// exact FP64 value of an output (zero or a normal number below 1): GB300's FP64 pipe is narrow
+__device__ __forceinline__ double fs_rl_f2d(float x)
+{
+    const fs_u32 u = __float_as_uint(x);
+    return __hiloint2double((int)(u ? (u >> 3) + (896u << 20) : 0u), (int)(u << 29));
+}
+
 // ranluxcl64 (pyopencl-ranluxcl.cl:893-920) with the same four-value buffering
 template <int NSKIP>
 struct FsRanluxStream64 {
@@ -541,8 +548,11 @@ struct FsRanluxStream64 {
         fs_rl_next4<NSKIP>(st, v0, v1, v2, v3);
         if (v0 == 0x1p-48f) v0 = 0.0f;
         if (v2 == 0x1p-48f) v2 = 0.0f;
-        a = __dadd_rn((double)v0, __ddiv_rn((double)v1, 16777216.0));
-        b = __dadd_rn((double)v2, __ddiv_rn((double)v3, 16777216.0));
+        // v0 + v1 / 2^24, the exact quotient rounded into the sum: one FP64 operation where a
+        // division takes about ten, and the conversions on the integer pipe (five atoms in FP64, 1024
+        // walkers, 4 sweeps: 3333 -> 3268 us)
+        a = __fma_rn(fs_rl_f2d(v1), 0x1p-24, fs_rl_f2d(v0));
+        b = __fma_rn(fs_rl_f2d(v3), 0x1p-24, fs_rl_f2d(v2));
     }
 
     __device__ __forceinline__ double next()
