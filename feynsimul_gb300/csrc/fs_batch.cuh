@@ -29,12 +29,10 @@ __device__ __forceinline__ fs_u32 fsb_offset(FsbStream &g, fs_u32 range)
 {
     return ((fs_u32)__fmul_rn(g.next(), (float)range)) & (range - 1u);  // kernel.c:715-718, fixed mode
 }
-#define FSB_DRAW_UNROLL _Pragma("unroll 1")  // one inlined generator per move loop
 #else
 typedef FsXorshift FsbStream;
 __device__ __forceinline__ float fsb_uniform(FsbStream &g) { return fs_xs_float(g); }
 __device__ __forceinline__ fs_u32 fsb_offset(FsbStream &g, fs_u32 range) { return fs_xs_next(g) & (range - 1u); }
-#define FSB_DRAW_UNROLL _Pragma("unroll")
 #endif
 
 struct FsBatchSys {
@@ -225,17 +223,33 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
                         const int m = ((1 + 2 * i) * half + start) & (N - 1);
                         const int l = (i * 2 * half + start) & (N - 1);
                         const int r = ((i + 1) * 2 * half + start) & (N - 1);
-                        FSB_DRAW_UNROLL
-                        for (int d = 0; d < DOF; d++) {
-                            const float u = fsb_uniform(g);
-                            const float v = fsb_uniform(g);
-                            // evaluated for every degree of freedom and replaced by 0 where
-                            // v == 0 (kernel.c:349-353): no branch, so the compiler
-                            // interleaves the degrees of freedom
+                        // Box-Muller evaluated for every degree of freedom and replaced by 0
+                        // where v == 0 (kernel.c:349-353): no branch, so the compiler interleaves
+                        // the degrees of freedom
+                        auto node_x = [&](int d, float u, float v) {
                             float rz = __fmul_rn(__fmul_rn(sig, sqrtf(__fmul_rn(-2.f, __logf(v)))),
                                                  __sinf(__fmul_rn(6.28318548f, u)));
                             rz = v != 0.f ? rz : 0.f;
                             FSB_AT(P, d, m) = __fadd_rn(__fmul_rn(0.5f, __fadd_rn(FSB_AT(P, d, l), FSB_AT(P, d, r))), rz);
+                        };
+#if FSB_RANLUX
+                        // twelve values at a time, as the sweep's moves
+#pragma unroll 1
+                        for (int d0 = 0; d0 + 6 <= DOF; d0 += 6) {
+                            float uv[12];
+                            g.template next_k<12>(uv);
+#pragma unroll
+                            for (int d = 0; d < 6; d++) node_x(d0 + d, uv[2 * d], uv[2 * d + 1]);
+                        }
+#pragma unroll 1
+                        for (int d = DOF / 6 * 6; d < DOF; d++) {
+#else
+#pragma unroll
+                        for (int d = 0; d < DOF; d++) {
+#endif
+                            const float u = fsb_uniform(g);
+                            const float v = fsb_uniform(g);
+                            node_x(d, u, v);
                         }
                     }
                 }

@@ -326,6 +326,30 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
             const fs_u32 m = ((fs_u32)((1 + 2 * i) * half) + start) & (FS_N - 1);
             const fs_u32 l = ((fs_u32)(i * 2 * half) + start) & (FS_N - 1);
             const fs_u32 r = ((fs_u32)((i + 1) * 2 * half) + start) & (FS_N - 1);
+#if FS_RANLUX && !FS_DOUBLE && FS_DOF > 8 && FS_MINB * FS_BLOCK <= 640
+            // the node's uniforms twelve at a time (u, v of six degrees), the rest one by one: less
+            // bookkeeping and six independent log / sqrt / sin chains (5 atoms, N = 128, 4000 walkers:
+            // 454 -> 377 us a run; 10 atoms, N = 256: 1137 -> 1021).  Not under a register budget of
+            // 64, where the twelve values spill (10 atoms, N = 1024 in device memory: 3830 against 3920)
+            auto node_x = [&](int d, float u, float v) {
+                float rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(FS_MUL((FT)FS_TWO_PI, u)));
+                rz = v != 0.0f ? rz : 0.0f;
+                FS_AT(P, d, m) = FS_ADD(FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r))), rz);
+            };
+#pragma unroll 1
+            for (int d0 = 0; d0 + 6 <= FS_DOF; d0 += 6) {
+                float uv[12];
+                g.template next_k<12>(uv);
+#pragma unroll
+                for (int d = 0; d < 6; d++) node_x(d0 + d, uv[2 * d], uv[2 * d + 1]);
+            }
+#pragma unroll 1
+            for (int d = FS_DOF / 6 * 6; d < FS_DOF; d++) {
+                const float u = fs_uniform(g);
+                const float v = fs_uniform(g);
+                node_x(d, u, v);
+            }
+#else
 #if FS_RANLUX && !FS_DOUBLE && (2 * FS_DOF) % 4 == 0
             // the node's 2*DOF uniforms (u, v per degree) in whole generator calls
             float uv[2 * FS_DOF];
@@ -362,6 +386,7 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
                 rz = v != (FT)0 ? rz : (FT)0;
                 FS_AT(P, d, m) = FS_ADD(FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r))), rz);
             }
+#endif
         }
     }
     FT aNew = (FT)0;

@@ -1,4 +1,5 @@
-"""The sweep's twelve-value RANLUX draws (six degrees of freedom) against the oracle: the
+"""The sweep's twelve-value RANLUX draws (six degrees of freedom; more in groups of six and a
+remainder drawn one by one) against the oracle: the
 generator tables bit-exact after every launch, for every luxury and from every position that
 a launch can end at.  A move of S = 2 draws 37 values and one of S = 1 draws 13, so the
 starting quad, the buffered values and the place of the skip inside a draw run through all
@@ -19,13 +20,13 @@ def _gpu():
     require_gpu()
 
 
-@pytest.mark.parametrize("S", [1, 2])
-@pytest.mark.parametrize("lux", [0, 1, 2, 3, 99, 123])
-def test_tables_match_oracle(lux, S):
+@pytest.mark.parametrize("dof,lux,S", [(6, lux, S) for lux in (0, 1, 2, 3, 99, 123) for S in (1, 2)]
+                         + [(9, 2, 1), (9, 1, 2), (12, 3, 1), (15, 2, 2)])
+def test_tables_match_oracle(dof, lux, S):
     from oracle import oracle as orc
     kernel, kernel_args = engine()
-    pot = "0.5 * (" + " + ".join(f"x{d + 1} * x{d + 1}" for d in range(6)) + ")"
-    system = types.SimpleNamespace(DOF=6, potential=pot, userCode="")
+    pot = "0.5 * (" + " + ".join(f"x{d + 1} * x{d + 1}" for d in range(dof)) + ")"
+    system = types.SimpleNamespace(DOF=dof, potential=pot, userCode="")
     W, N = 6, 16
     ka = kernel_args.KernelArgs(
         system=system, nbrOfWalkers=W, N=N, beta=2.0, S=S, enableOperator=True, enableCorrelator=False,
@@ -37,7 +38,7 @@ def test_tables_match_oracle(lux, S):
     k.initRanlux()
     k.groupInitRanlux()
     o = orc.OracleSampler(orc.OracleConfig(
-        DOF=6, potential=pot, userCode="", nbrOfWalkers=W, N=N, beta=2.0, S=S, operatorRuns=3,
+        DOF=dof, potential=pot, userCode="", nbrOfWalkers=W, N=N, beta=2.0, S=S, operatorRuns=3,
         metroStepsPerOperatorRun=3, nbrOfWalkersPerWorkGroup=1, enableParallelizePath=True, enableRanlux=True,
         luxuaryFactor=lux, ranluxIntMax=2 ** 32 - 1, operators=("x1 * x6",), compat=False, accum=1))
     p0 = (np.random.RandomState(3).randn(*o.paths.shape) * 0.4).astype(np.float32)
