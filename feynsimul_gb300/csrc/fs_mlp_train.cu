@@ -395,14 +395,14 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
                 for (int o = 0; o < 16; o++) put(out + P_W4 + o * 128 + r, v[o]);
             }
         }
-        auto quarters = [&](int i) { return (S.db[0][i] + S.db[1][i]) + (S.db[2][i] + S.db[3][i]); };
+        auto quarters = [&](int i) { return ((S.db[0][i] + S.db[1][i]) + S.db[2][i]) + S.db[3][i]; };
         if (tid < 128) {
             put(out + P_B1 + tid, quarters(tid));
             put(out + P_B2 + tid, quarters(128 + tid));
             put(out + P_B3 + tid, quarters(256 + tid));
         }
         if (tid < 16) put(out + P_B4 + tid, quarters(384 + tid));
-        const float loss = (S.loss[0] + S.loss[1]) + (S.loss[2] + S.loss[3]);
+        const float loss = ((S.loss[0] + S.loss[1]) + S.loss[2]) + S.loss[3];
         if (tid == 0 && part) out[FS_MLP_NPARAM] = loss;
         if (tid == 0 && !part && loss_out) atomicAdd(loss_out, loss);
     }
@@ -448,9 +448,8 @@ __global__ void fs_mlp_adam_kernel(float *params, float *m, float *v, float *gra
     grad[i] = 0.f;
 }
 
-// Adam step on the gradient that n_parts CTAs of the training pass left in their rows of part:
-// added in order with the rounding errors on the side (TwoSum), so the sum is the exact one
-// rounded once or twice, and the same whenever the rows are.  The last thread adds the losses.
+// Adam step on the gradient that n_parts CTAs of the training pass left in their rows of part,
+// added in the CTAs' order.  The last thread adds the losses.
 __global__ void fs_mlp_adam_parts_kernel(const float *__restrict__ part, int n_parts, float *params, float *m, float *v,
                                          fs_bf16 *wq, float lr, float b1c, float b2c, float *loss_out)
 {
@@ -463,16 +462,9 @@ __global__ void fs_mlp_adam_parts_kernel(const float *__restrict__ part, int n_p
     else if (i >= P_W3 && i < P_B3) p = P_W3 + (i - P_W3) % 512 / 4 * 128 + (i - P_W3) / 512 * 4 + i % 4;
     const bool param = i < FS_MLP_NPARAM;
     const float w0 = param ? params[p] : 0.f, m0 = param ? m[p] : 0.f, v0 = param ? v[p] : 0.f;
-    float s = 0.f, e = 0.f;
+    float g = 0.f;
 #pragma unroll 16
-    for (int k = 0; k < n_parts; k++) {
-        const float x = part[(size_t)k * TT_PART + i];
-        const float t = __fadd_rn(s, x);
-        const float bp = __fsub_rn(t, s);
-        e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, bp)), __fsub_rn(x, bp)));
-        s = t;
-    }
-    const float g = __fadd_rn(s, e);
+    for (int k = 0; k < n_parts; k++) g = __fadd_rn(g, part[(size_t)k * TT_PART + i]);
     if (param) adam_one(p, g, w0, m0, v0, params, m, v, wq, lr, b1c, b2c);
     else if (loss_out) *loss_out = g;
 }

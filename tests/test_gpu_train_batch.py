@@ -61,8 +61,8 @@ def test_batch_matches_pass_and_repeats(rows, dof):
     parts = work.cpu().numpy().astype(np.float64).reshape(n_parts, stride)[:, :p.size + 1]
     magnitude = np.abs(parts).sum(axis=0)
     u = 2.0 ** -24
-    # the ordered sum with its errors on the side, then 0.1 * g: four roundings at most
-    assert abs(float(loss[0]) - parts[:, -1].sum()) <= 4 * u * magnitude[-1]
+    # the ordered sum of the CTAs' losses
+    assert abs(float(loss[0]) - parts[:, -1].sum()) <= n_parts * u * magnitude[-1]
     # the pass over copied rows: the same partial gradients, added by atomics in FP32
     tg = torch.zeros_like(tp)
     l2 = torch.zeros(1, dtype=torch.float32, device="cuda")
@@ -78,6 +78,6 @@ def test_batch_matches_pass_and_repeats(rows, dof):
     for at, k in ((0, 16), (2048 + 128, 128), (2048 + 128 + 16384 + 128, 128)):
         block = mag[at:at + 128 * k].reshape(k // 4, 128, 4)
         mag[at:at + 128 * k] = block.transpose(1, 0, 2).reshape(-1)
-    assert np.all(np.abs(g - want) <= (n_parts + 8) * u * mag)
-    assert abs(float(loss[0]) - float(l2[0])) <= (n_parts + 8) * u * magnitude[-1]
+    assert np.all(np.abs(g - want) <= (2 * n_parts + 8) * u * mag)
+    assert abs(float(loss[0]) - float(l2[0])) <= (2 * n_parts + 8) * u * magnitude[-1]
     assert np.abs(want).max() > 0
