@@ -67,6 +67,7 @@ struct fs_handle {
     std::vector<std::string> ops, cors, hists;
     // launch geometry
     int tpw = 1, seg = 1, wpb = 1, block = 1, grid = 1;
+    int lanes = 1;  // lanes that share a segment thread (FS_G)
     int cor_ilv = 0;  // correlator lags summed in one slice pass over a doubled slice buffer
     int pipe = 0;     // correlator helpers one measurement behind the movers (FS_PIPE)
     long long snstride = 0;  // FS_PIPE: one path snapshot in shared memory, elements
@@ -338,7 +339,7 @@ static std::string gen_source(const fs_handle &h, const std::string &potential,
       << "\n#define FS_VCACHE " << (h.vstride || h.vglobal ? 1 : 0) << "\n#define FS_VSTRIDE " << h.vstride
       << "\n#define FS_VGLOBAL " << h.vglobal
       << "\n#define FS_COR_ILV " << h.cor_ilv << "\n#define FS_CWSTRIDE " << h.cwstride << "\n#define FS_MX "
-      << h.mx << "\n#define FS_PIPE " << h.pipe << "\n#define FS_SNSTRIDE " << h.snstride << "\n";
+      << h.mx << "\n#define FS_PIPE " << h.pipe << "\n#define FS_SNSTRIDE " << h.snstride << "\n#define FS_G " << h.lanes << "\n";
     {
         const int mv = c.moves ? c.moves : FS_MOVE_BISECTION;
         const double nb = (double)c.n_slices / c.beta;
@@ -564,13 +565,51 @@ static size_t sweep_smem(const fs_handle &h, long long vstride, size_t hist_byte
 // the instruction cache (5 atoms: 634 at 4, 824 at one).
 static int default_wpb(const fs_handle &h, size_t per_walker, size_t hist_bytes)
 {
-    if (h.tpw > 32) return 1;
-    int wpb = std::max(1, (h.tpw == 1 ? 32 : 128) / h.tpw);
+    const int lpw = h.tpw * h.lanes;
+    if (lpw > 32) return 1;
+    int wpb = std::max(1, (lpw == 1 ? 32 : 128) / lpw);
     while (wpb > 1 && per_walker * wpb + hist_bytes > 100 * 1024) wpb /= 2;
-    const bool single = h.tpw == 1, cheap = h.cfg.dof <= 2;
+    const bool single = lpw == 1, cheap = h.cfg.dof <= 2;
     const int least = !single ? 32 : cheap ? 1 : 4, ctas = single && cheap ? 4 * device_sms() : device_sms();
-    while (wpb * h.tpw > least && (h.cfg.n_walkers + wpb - 1) / wpb < ctas) wpb /= 2;
+    while (wpb * lpw > least && (h.cfg.n_walkers + wpb - 1) / wpb < ctas) wpb /= 2;
     return wpb;
+}
+
+// Lanes that share a segment thread (FS_G in fs_pimc.cuh).  A run of few walkers leaves most
+// schedulers without a warp, and a segment thread's move is one serial chain: the draws, then every
+// degree's Box-Muller values, then every slice's potential.  Lanes that repeat the draws and share
+// the rest shorten it until the chip is full, i.e. up to about two warps per scheduler; the
+// repeated draws cost more with RANLUX, and moves that are slow for other reasons (IEEE functions,
+// the narrow FP64 pipe) bear more lanes.  Measured, us a run for 1 / 2 / 4 / 8 lanes (608
+// schedulers; one-lane warps in brackets): bound trimer IEEE (111) 459 / 286 / 214 / 197, (300) 460 /
+// 289 / 251 / 294, (600) 473 / 343 / 392 / 563, (1250) 724 / 721 / 906 / 1112; fast (10) 155 / 112 / 113
+// / 95, (111) 157 / 113 / 113 / 130, (300) 159 / 115 / 145 / 211, (600) 167 / 164 / 238 / 381, (1250) 311 /
+// 388 / - / -; trimer RANLUX (50) 136 / 116 / 103 / 101, (150) 136 / 116 / 104 / 125, (300) 121 / 105 / 106
+// / 149, (600) 141 / 146 / 207 / 360; 10 atoms (150) 398 / 188 / 127 / 125, (1000) 202 / 286 / 247 / 247;
+// 5 atoms FP64 (50) 4676 / 2855 / 1619 / 1194, (200) 4678 / 3225 / 2324 / 2638, (512) 5170 / 5520 / 4551 /
+// 5653.  With segments of 4 slices a trimer's lanes have too little to share (T = 64: 51 / 56 / 67,
+// FP64 749 / 480 / 545).  Twelve-value RANLUX draws need at most 8 degrees of freedom here, and
+// potentials of one or two degrees have nothing to share.
+static int lanes_for(const fs_handle &h)
+{
+    const fs_config &c = h.cfg;
+    const bool dbl = c.enable_double != 0, ranlux = c.enable_ranlux != 0;
+    if (!c.enable_parallelize_path || !h.cors.empty() || c.learned || c.walkers_per_block > 0 || c.dof < 3 ||
+        h.seg > 32 || (ranlux && !dbl && (c.dof > 8 || c.dof % 2)))
+        return 1;
+    const double warps = (double)h.n_threads / 32, schedulers = 4.0 * device_sms();
+    const struct {
+        int lanes;
+        double most;  // warps per scheduler with them
+    } rule[] = {{8, dbl || !c.fast_math ? 1.5 : 0.66},
+                {4, dbl ? 3.4 : !c.fast_math ? 2.0 : 1.0},
+                {2, dbl ? 1.0 : ranlux ? 1.6 : 2.0}};
+    for (const auto &r : rule) {
+        if (r.lanes > h.seg || r.lanes * h.tpw > 1024 || warps * r.lanes > r.most * schedulers) continue;
+        if (c.dof <= 8 && (r.lanes > h.seg / 2 || (h.seg < 8 && r.lanes * h.tpw > 32))) continue;
+        return r.lanes;
+    }
+    return 1;
 }
 
 // The reference's enableGlobalPath says where its kernel keeps the paths; the results are the
@@ -589,9 +628,9 @@ static bool path_in_shared(const fs_handle &h, size_t path_bytes, size_t hist_by
                              c.n_walkers);
     const size_t smem = path_bytes * wpb + 2 * 16 * h.ft + hist_bytes;
     if (smem > 227 * 1024) return false;
-    const long long ctas = std::min((227ll * 1024) / (long long)(smem + 1024), 2048ll / (wpb * h.tpw));
+    const long long ctas = std::min((227ll * 1024) / (long long)(smem + 1024), 2048ll / (wpb * h.tpw * h.lanes));
     if (ctas < std::max(1, c.min_blocks_per_sm)) return false;
-    return ctas * device_sms() * wpb >= c.n_walkers || ctas * wpb * h.tpw >= 384;
+    return ctas * device_sms() * wpb >= c.n_walkers || ctas * wpb * h.tpw * h.lanes >= 384;
 }
 
 static int validate(const fs_config &c, int nops, int ncor, int nhist)
@@ -741,6 +780,7 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
     h->tpw = c.enable_parallelize_path ? (c.n_slices >> c.bisection_level) : 1;
     h->n_threads = (long long)c.n_walkers * h->tpw;
     h->ft = c.enable_double ? 8 : 4;
+    h->lanes = lanes_for(*h);
     {
         // FP32-partial correlator sums (every mode but the reference's FP32 order, FP32
         // builds) with at most 4 lags per thread run every lag in one pass over the slice
@@ -798,7 +838,7 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
     // two banks: 60000 oscillators in walker mode took 1486 us a run, 1178 with this).
     const long long dstride = c.n_slices + (c.n_slices >> c.bisection_level);
     auto spread = [&](long long words) {
-        if (h->tpw >= 32) return round16(words);
+        if (h->tpw * h->lanes >= 32) return round16(words);
         const long long want = (h->tpw * ((1ll << c.bisection_level) + 1)) % 32;
         return words + (want - words % 32 + 32) % 32;
     };
@@ -852,7 +892,7 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         }
         while (c.n_walkers % h->wpb) h->wpb -= wpw;
     }
-    h->block = h->wpb * h->tpw * h->mx;
+    h->block = h->wpb * h->tpw * h->lanes * h->mx;
     if (h->block > 1024) {
         delete h;
         return fail(nullptr, FS_ERR_CONFIG, "walkers_per_block * threads per walker exceeds 1024");

@@ -44,7 +44,19 @@
 #ifndef FS_SNSTRIDE
 #define FS_SNSTRIDE 0
 #endif
-#define FS_MBLOCK (FS_WPB * FS_TPW)          // threads that run the moves
+// Lanes per segment thread (FS_G, 1 unless the host finds the run too small to fill the chip):
+// FS_G neighbouring lanes share one reference work-item.  Each advances its own identical copy of
+// the generator, draws the proposals of every FS_G-th degree of freedom and evaluates the
+// potential and the operators of every FS_G-th slice; the sums are formed from the lanes' values
+// in the same order, so the results are the same bit for bit.
+#ifndef FS_G
+#define FS_G 1
+#endif
+#define FS_LPW (FS_TPW * FS_G)               // lanes per walker
+#if FS_G > 1 && (!FS_PARALLEL || FS_NCOR > 0 || FS_LEARNED || FS_MX > 1 || FS_SEG % FS_G != 0 || FS_SEG > 32)
+#error "lanes sharing a segment thread need parallel-path mode, segments of FS_G to 32 slices and no correlators"
+#endif
+#define FS_MBLOCK (FS_WPB * FS_LPW)          // threads that run the moves
 #define FS_BLOCK (FS_MBLOCK * FS_MX)
 #define FS_CTPW (FS_TPW * (FS_MX - FS_PIPE))  // correlator threads per walker
 #if FS_PIPE
@@ -431,6 +443,131 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
     return 1;
 }
 
+#if FS_G > 1
+// lane j's value, from the lanes of this segment thread
+__device__ __forceinline__ FT fs_from_lane(FT v, int j)
+{
+    const unsigned first = (threadIdx.x & 31u) & ~(FS_G - 1u);
+    return __shfl_sync(((1u << FS_G) - 1u) << first, v, first + j);
+}
+
+// fs_bisect shared by the FS_G lanes of a segment thread: lane gl proposes the degrees of freedom
+// gl, gl + FS_G, ... of every node (the levels of one degree need no other's values) and
+// evaluates the potential at the slices gl + 1, gl + 1 + FS_G, ...; all lanes draw the same
+// uniforms, form the same sums in slice order and take the same decision.
+#define FS_DPL ((FS_DOF + FS_G - 1) / FS_G)   // degrees of freedom of a lane
+#if FS_FAST || FS_DPL <= 2
+#define FS_LANE_UNROLL _Pragma("unroll")
+#else
+#define FS_LANE_UNROLL _Pragma("unroll 1")
+#endif
+__device__ __forceinline__ int fs_bisect_lanes(FT *P, FT *Vc, fs_u32 start, FsUStream &g, const FT *sigma, int gl)
+{
+    FT old[FS_DPL][FS_SEG - 1];
+#pragma unroll
+    for (int k = 0; k < FS_DPL; k++) {
+        const int d = min(k * FS_G + gl, FS_DOF - 1);
+#pragma unroll
+        for (int i = 1; i < FS_SEG; i++) old[k][i - 1] = FS_AT(P, d, (start + (fs_u32)i) & (FS_N - 1));
+    }
+    // V of this lane's slices, and the action of the lanes' values in slice order
+    FT own[FS_SEG / FS_G], was[FS_SEG / FS_G];
+    auto potentials = [&](FT (&v)[FS_SEG / FS_G]) {
+        FS_ACT_UNROLL
+        for (int k = 0; k < FS_SEG / FS_G; k++) {
+            const int i = k * FS_G + gl + 1;
+            const fs_u32 p = (start + (fs_u32)i) & (FS_N - 1);
+            if (i < FS_SEG) own[k] = fs_pot(FS_ARGS_AT(P, p));
+        }
+#pragma unroll
+        for (int k = 0; k < FS_SEG / FS_G; k++) v[k] = own[k];
+    };
+    auto action = [&](const FT (&v)[FS_SEG / FS_G]) {
+        FT s = (FT)0;
+#pragma unroll
+        for (int i = 1; i < FS_SEG; i++)
+            s = FS_ADD(s, FS_MUL((FT)FS_EPS, fs_from_lane(v[(i - 1) / FS_G], (i - 1) % FS_G)));
+        return s;
+    };
+#pragma unroll
+    for (int k = 0; k < FS_SEG / FS_G; k++) own[k] = (FT)0;
+#if FS_VCACHE
+#pragma unroll
+    for (int k = 0; k < FS_SEG / FS_G; k++) {
+        const int i = k * FS_G + gl + 1;
+        was[k] = i < FS_SEG ? Vc[FS_VIDX((start + (fs_u32)i) & (FS_N - 1))] : (FT)0;
+    }
+#else
+    (void)Vc;
+    potentials(was);
+#endif
+    const FT aOld = action(was);
+#pragma unroll 1
+    for (int n = 1; n <= FS_S; n++) {
+        const int half = 1 << (FS_S - n);
+        const FT sig = sigma[n];
+#pragma unroll 1
+        for (int i = 0; i < (1 << (n - 1)); i++) {
+            const fs_u32 m = ((fs_u32)((1 + 2 * i) * half) + start) & (FS_N - 1);
+            const fs_u32 l = ((fs_u32)(i * 2 * half) + start) & (FS_N - 1);
+            const fs_u32 r = ((fs_u32)((i + 1) * 2 * half) + start) & (FS_N - 1);
+#if FS_RANLUX && !FS_DOUBLE
+            float uv[2 * FS_DOF];
+            g.template next_k<2 * FS_DOF>(uv);
+#pragma unroll
+#else
+            FS_LANE_UNROLL
+#endif
+            for (int k = 0; k < FS_DPL; k++) {
+                FT u = (FT)0, v = (FT)0;
+#pragma unroll
+                for (int j = 0; j < FS_G; j++) {
+                    if (FS_DOF % FS_G != 0 && k * FS_G + j >= FS_DOF) break;
+#if FS_RANLUX && !FS_DOUBLE
+                    const FT uj = uv[2 * (k * FS_G + j)], vj = uv[2 * (k * FS_G + j) + 1];
+#else
+                    const FT uj = fs_uniform(g);
+                    const FT vj = fs_uniform(g);
+#endif
+                    u = j == gl ? uj : u;
+                    v = j == gl ? vj : v;
+                }
+                const int d = k * FS_G + gl;
+                FT rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(FS_MUL((FT)FS_TWO_PI, u)));
+                rz = v != (FT)0 ? rz : (FT)0;
+                if (FS_DOF % FS_G == 0 || d < FS_DOF)
+                    FS_AT(P, d, m) = FS_ADD(FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r))), rz);
+            }
+        }
+    }
+    const unsigned first = (threadIdx.x & 31u) & ~(FS_G - 1u), group = ((1u << FS_G) - 1u) << first;
+    __syncwarp(group);  // every degree's new nodes
+    FT now[FS_SEG / FS_G];
+    potentials(now);
+    const FT aNew = action(now);
+    const FT acc = fs_uniform(g);
+    const bool reject = FS_EXP(FS_SUB(aOld, aNew)) < acc;
+    __syncwarp(group);  // the lanes have read the new nodes before one puts the old ones back
+    if (reject) {
+#pragma unroll
+        for (int k = 0; k < FS_DPL; k++)
+            if (FS_DOF % FS_G == 0 || k * FS_G + gl < FS_DOF)
+#pragma unroll
+                for (int i = 1; i < FS_SEG; i++)
+                    FS_AT(P, k * FS_G + gl, (start + (fs_u32)i) & (FS_N - 1)) = old[k][i - 1];
+        return 0;
+    }
+#if FS_VCACHE
+#pragma unroll
+    for (int k = 0; k < FS_SEG / FS_G; k++) {
+        const int i = k * FS_G + gl + 1;
+        if (i < FS_SEG) Vc[FS_VIDX((start + (fs_u32)i) & (FS_N - 1))] = now[k];
+    }
+#endif
+    return 1;
+}
+#endif
+
 #ifndef FS_BISECT
 #define FS_BISECT 1
 #endif
@@ -745,9 +882,11 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 
     const int tid_b = threadIdx.x;
     const int grp = tid_b / FS_MBLOCK;             // 0: movers; 1..FS_MX-1: correlator helpers
-    const int wl = (tid_b - grp * FS_MBLOCK) / FS_TPW;
-    const int t = tid_b % FS_TPW;
+    const int wl = (tid_b - grp * FS_MBLOCK) / FS_LPW;
+    const int t = tid_b % FS_LPW / FS_G;
+    const int gl = FS_G > 1 ? tid_b % FS_G : 0;    // lane of the segment thread
     const bool mover = FS_MX == 1 || grp == 0;
+    const bool owner = mover && gl == 0;           // writes the work-item's state back
     // this thread's lags FS_LAG(j): lt + j * FS_CTPW; with FS_PIPE the helper lanes lt < N/8
     // own lags 4 lt + j
     const int lt = (grp - FS_PIPE) * FS_TPW + t;
@@ -796,10 +935,10 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #else
 #define FS_WSYNC() do { if (mover) asm volatile("bar.sync 1, %0;" ::"n"(FS_MBLOCK) : "memory"); } while (0)
 #endif
-#elif FS_TPW <= 32 && FS_MX == 1
+#elif FS_LPW <= 32 && FS_MX == 1
         const unsigned lane = threadIdx.x & 31u;
-        const unsigned wmask = FS_TPW == 32 ? 0xFFFFFFFFu
-                                            : (((1u << FS_TPW) - 1u) << (lane / FS_TPW * FS_TPW));
+        const unsigned wmask = FS_LPW == 32 ? 0xFFFFFFFFu
+                                            : (((1u << FS_LPW) - 1u) << (lane / FS_LPW * FS_LPW));
 #define FS_WSYNC() __syncwarp(wmask)
 #else
 #define FS_WSYNC() __syncthreads()
@@ -828,7 +967,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
         // The walker's offset stream: every reference work-item of the walker advances an
         // identical copy; here one lane advances it in shared memory for the walker.
         FsIStream &is = s_istream[wl];
-        if (mover && t == 0) {
+        if (owner && t == 0) {
 #if FS_COMPAT
             fs_rl_load<FS_NSKIP>(is.st, a.gtab + (size_t)tid * 28);
 #else
@@ -899,16 +1038,14 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
             const int v_lo = 0, v_hi = FS_N;
 #endif
 #pragma unroll 1
-            for (int s = v_lo; s < (mover ? v_hi : v_lo); s++) Vc[FS_VIDX(s)] = fs_pot(FS_ARGS_AT(P, s));
+            for (int s = v_lo + gl; s < (mover ? v_hi : v_lo); s += FS_G) Vc[FS_VIDX(s)] = fs_pot(FS_ARGS_AT(P, s));
         }
         FS_WSYNC();
 #endif
 
 #if FS_NOPS > 0
-        // the operators of a slice's coordinates, added to this thread's sums
-        auto fs_op_add = [&](const FT *x) {
-            FT ov[FS_NOPS];
-            fs_ops(FS_ARGS_OF(x), ov);
+        // a slice's operator values, added to this thread's sums
+        auto fs_op_add = [&](const FT *ov) {
 #pragma unroll
             for (int i = 0; i < FS_NOPS; i++) {
 #if FS_ACCUM == 0
@@ -1272,7 +1409,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #if FS_OFF_PRE
                 const fs_u32 off = s_offs[wl][run * FS_MSTEPS + step];
 #else
-                if (mover && t == 0) s_off[wl] = fs_offset(is, FS_PARALLEL ? FS_SEG : FS_N);
+                if (owner && t == 0) s_off[wl] = fs_offset(is, FS_PARALLEL ? FS_SEG : FS_N);
                 FS_WSYNC();
                 const fs_u32 off = s_off[wl];
 #endif
@@ -1314,7 +1451,11 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
                 }
                 n_acc += (fs_u32)fs_bisect(P, Vc, start, fs, sigma, lmu, lsd);
 #else
+#if FS_G > 1
+                n_acc += (fs_u32)fs_bisect_lanes(P, Vc, start, fs, sigma, gl);
+#else
                 if (mover) n_acc += (fs_u32)fs_bisect(P, Vc, start, fs, sigma, nullptr, nullptr);
+#endif
 #endif
 #endif  // FS_BISECT
                 FS_WSYNC();
@@ -1325,6 +1466,55 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #else
             const int s_lo = 0, s_hi = FS_N;
 #endif
+            // counts of a slice's coordinates
+            auto fs_count = [&](const FT *x) {
+                (void)x;
+#if FS_BINS
+                {
+                    int ok = 1, inc = 1, bi = 0;
+#pragma unroll
+                    for (int d = 0; d < FS_DOF; d++) {
+                        if (x[d] < (FT)FS_XMIN || x[d] >= (FT)FS_XMAX) ok = 0;
+                        bi += (int)((fs_u32)FS_MUL(FS_SUB(x[d], (FT)FS_XMIN), (FT)FS_INVBIN)) * inc;
+                        inc *= FS_BINRES;
+                    }
+                    if (ok) atomicAdd(a.bins + bi, 1u);
+                }
+#endif
+#if FS_NHIST > 0
+                {
+                    FT hv[FS_NHIST];
+                    fs_hist(FS_ARGS_OF(x), hv);
+#pragma unroll
+                    for (int h = 0; h < FS_NHIST; h++) {
+                        if (hv[h] >= (FT)FS_HLO && hv[h] < (FT)FS_HHI) {
+                            const int k = (int)FS_MUL(FS_SUB(hv[h], (FT)FS_HLO), (FT)FS_HINVW);
+                            if (k >= 0 && k < FS_HBINS) atomicAdd(s_hist + k, 1u);
+                        }
+                    }
+                }
+#endif
+            };
+#if FS_G > 1
+#pragma unroll 1
+            for (int s0 = s_lo; s0 < s_hi; s0 += FS_G) {
+                FT x[FS_DOF];
+#pragma unroll
+                for (int d = 0; d < FS_DOF; d++) x[d] = FS_AT(P, d, s0 + gl);
+#if FS_NOPS > 0
+                FT ov[FS_NOPS];
+                fs_ops(FS_ARGS_OF(x), ov);
+#pragma unroll
+                for (int j = 0; j < FS_G; j++) {
+                    FT oj[FS_NOPS];
+#pragma unroll
+                    for (int i = 0; i < FS_NOPS; i++) oj[i] = fs_from_lane(ov[i], j);
+                    fs_op_add(oj);
+                }
+#endif
+                fs_count(x);
+            }
+#else
 #pragma unroll 1
             for (int s0 = s_lo; s0 < (mover ? s_hi : s_lo); s0 += FS_MEAS_BATCH) {
                 FT xb[FS_MEAS_BATCH][FS_DOF];
@@ -1338,7 +1528,9 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
                     const FT *x = xb[b];
                     (void)s;
 #if FS_NOPS > 0
-                    fs_op_add(x);
+                    FT ov[FS_NOPS];
+                    fs_ops(FS_ARGS_OF(x), ov);
+                    fs_op_add(ov);
 #endif
 #if FS_PIPE
 #pragma unroll
@@ -1346,33 +1538,10 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #elif FS_NCOR > 0
                     fs_cor_put(x, s);
 #endif
-#if FS_BINS
-                    {
-                        int ok = 1, inc = 1, bi = 0;
-#pragma unroll
-                        for (int d = 0; d < FS_DOF; d++) {
-                            if (x[d] < (FT)FS_XMIN || x[d] >= (FT)FS_XMAX) ok = 0;
-                            bi += (int)((fs_u32)FS_MUL(FS_SUB(x[d], (FT)FS_XMIN), (FT)FS_INVBIN)) * inc;
-                            inc *= FS_BINRES;
-                        }
-                        if (ok) atomicAdd(a.bins + bi, 1u);
-                    }
-#endif
-#if FS_NHIST > 0
-                    {
-                        FT hv[FS_NHIST];
-                        fs_hist(FS_ARGS_OF(x), hv);
-#pragma unroll
-                        for (int h = 0; h < FS_NHIST; h++) {
-                            if (hv[h] >= (FT)FS_HLO && hv[h] < (FT)FS_HHI) {
-                                const int k = (int)FS_MUL(FS_SUB(hv[h], (FT)FS_HLO), (FT)FS_HINVW);
-                                if (k >= 0 && k < FS_HBINS) atomicAdd(s_hist + k, 1u);
-                            }
-                        }
-                    }
-#endif
+                    fs_count(x);
                 }
             }
+#endif
 #if FS_NOPS > 0
             if (mover) fs_op_flush();
 #endif
@@ -1388,10 +1557,10 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
         }
 
         // ---- epilogue (kernel.c:801-836) ----
-        if (mover) a.accepts[tid] = n_acc;
+        if (owner) a.accepts[tid] = n_acc;
 #if FS_NOPS > 0
 #pragma unroll
-        for (int i = 0; i < (mover ? FS_NOPS : 0); i++) {
+        for (int i = 0; i < (owner ? FS_NOPS : 0); i++) {
             const size_t o = (size_t)tid * FS_NOPS + i;
 #if FS_ACCUM == 0
             ((FT *)a.op_means)[o] = FS_MUL(opr[i], (FT)FS_OPNORM);
@@ -1426,24 +1595,24 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #endif
             bool bad = false;
 #pragma unroll 1
-            for (int s = c_lo; s < c_hi; s++)
+            for (int s = c_lo + gl; s < c_hi; s += FS_G)
 #pragma unroll
                 for (int d = 0; d < FS_DOF; d++) bad |= !isfinite(FS_AT(P, d, s));
             if (bad) fs_flag_nonfinite(a.status, w);
         }
 #endif
 #if FS_RANLUX
-        if (mover) fs_rl_store<FS_NSKIP>(fs.st, a.rtab + (size_t)tid * 28);
+        if (owner) fs_rl_store<FS_NSKIP>(fs.st, a.rtab + (size_t)tid * 28);
         FS_WSYNC();
 #if FS_COMPAT
-        if (mover) fs_rl_store<FS_NSKIP>(is.st, a.gtab + (size_t)tid * 28);
+        if (owner) fs_rl_store<FS_NSKIP>(is.st, a.gtab + (size_t)tid * 28);
 #else
-        if (mover && t == 0) fs_rl_store<FS_NSKIP>(is.st, a.gtab + (size_t)w * 28);
+        if (owner && t == 0) fs_rl_store<FS_NSKIP>(is.st, a.gtab + (size_t)w * 28);
 #endif
 #else
-        if (mover) *(uint4 *)(a.seeds + (size_t)tid * 4) = make_uint4(fs.x, fs.y, fs.z, fs.w);
+        if (owner) *(uint4 *)(a.seeds + (size_t)tid * 4) = make_uint4(fs.x, fs.y, fs.z, fs.w);
 #if !FS_COMPAT
-        if (mover && t == 0) *(uint4 *)(a.walker_seeds + (size_t)w * 4) = make_uint4(is.x, is.y, is.z, is.w);
+        if (owner && t == 0) *(uint4 *)(a.walker_seeds + (size_t)w * 4) = make_uint4(is.x, is.y, is.z, is.w);
 #endif
 #endif
 #undef FS_WSYNC
