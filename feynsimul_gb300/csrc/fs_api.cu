@@ -69,6 +69,7 @@ struct fs_handle {
     int tpw = 1, seg = 1, wpb = 1, block = 1, grid = 1;
     int lanes = 1;  // lanes that share a segment thread (FS_G)
     int cor_ilv = 0;  // correlator lags summed in one slice pass over a doubled slice buffer
+    int plags = 4;    // lags a pipelined helper lane sums (FS_PLAGS)
     int pipe = 0;     // correlator helpers one measurement behind the movers (FS_PIPE)
     long long snstride = 0;  // FS_PIPE: one path snapshot in shared memory, elements
     int mx = 1;       // thread groups per CTA: 1 moving + mx - 1 summing correlator lags (FS_MX)
@@ -339,7 +340,7 @@ static std::string gen_source(const fs_handle &h, const std::string &potential,
       << "\n#define FS_VCACHE " << (h.vstride || h.vglobal ? 1 : 0) << "\n#define FS_VSTRIDE " << h.vstride
       << "\n#define FS_VGLOBAL " << h.vglobal
       << "\n#define FS_COR_ILV " << h.cor_ilv << "\n#define FS_CWSTRIDE " << h.cwstride << "\n#define FS_MX "
-      << h.mx << "\n#define FS_PIPE " << h.pipe << "\n#define FS_SNSTRIDE " << h.snstride << "\n#define FS_G " << h.lanes << "\n";
+      << h.mx << "\n#define FS_PIPE " << h.pipe << "\n#define FS_PLAGS " << h.plags << "\n#define FS_SNSTRIDE " << h.snstride << "\n#define FS_G " << h.lanes << "\n";
     {
         const int mv = c.moves ? c.moves : FS_MOVE_BISECTION;
         const double nb = (double)c.n_slices / c.beta;
@@ -793,13 +794,22 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         // movers copy their slices to a double-buffered path snapshot, and the helpers alone
         // evaluate the correlator values on it and sum the lags, one measurement behind the
         // moves.
-        // The pipelined helpers give each thread 4 consecutive lags (N/8 lag threads per
-        // walker) and sum FP32 partials over the doubled slice values.
+        // The pipelined helpers give each thread 4 or 2 consecutive lags (N/8 or N/4 lag threads
+        // per walker) and sum FP32 partials over the doubled slice values.
         if (!h->cors.empty() && c.enable_parallelize_path && !c.global_path && !c.learned && h->tpw <= 32) {
             const int lag_threads = std::min(c.n_slices / 2, 64);
             const int wpw = 32 / h->tpw;
             const int wpb_min = c.walkers_per_block > 0 ? c.walkers_per_block : wpw;
-            const int groups = (c.n_slices / 8 + h->tpw - 1) / h->tpw;
+            // 2 lags a lane where the lanes are there anyway (S <= 2: with 4 half of the helper threads
+            // are idle), or where every CTA has an SM to itself and a second group of helpers costs
+            // nothing: us a run of 40 sweeps, 4 / 2 lags: N = 64, S = 2, 1000 walkers 52 / 42, 4000 105 /
+            // 83; N = 128, S = 3, 256 walkers 52 / 44, 1024 68 / 69, 4096 163 / 190; N = 512, S = 4, 300
+            // walkers 150 / 179
+            auto groups_of = [&](int lags) { return (c.n_slices / (2 * lags) + h->tpw - 1) / h->tpw; };
+            if (groups_of(2) == groups_of(4) ||
+                (groups_of(2) == 2 && c.walkers_per_block == 0 && c.n_walkers / wpw <= device_sms()))
+                h->plags = 2;
+            const int groups = groups_of(h->plags);
             const bool fma_partials = (c.accum == FS_ACCUM_FP64 || c.accum == FS_ACCUM_KAHAN) &&
                                       !c.enable_double && c.partials == FS_PARTIALS_FP32;
             if (fma_partials && c.n_slices % 8 == 0 && c.n_slices >= 16 && h->tpw >= 2 && c.n_walkers % wpw == 0 &&
@@ -813,7 +823,7 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
             if (c.walkers_per_block > 0 && c.n_walkers % c.walkers_per_block) h->mx = 1, h->pipe = 0;
         }
         const long long lag_tpw = (long long)h->tpw * (h->mx - h->pipe);
-        const long long lpt = h->pipe ? 4 : (c.n_slices / 2 + lag_tpw - 1) / lag_tpw;
+        const long long lpt = h->pipe ? h->plags : (c.n_slices / 2 + lag_tpw - 1) / lag_tpw;
         h->cor_ilv = (c.accum != 0 && !c.enable_double && lpt <= 4) ? 1 : 0;
         // per-walker stride an odd multiple of 64 bytes: two walkers sharing a warp read
         // opposite bank halves

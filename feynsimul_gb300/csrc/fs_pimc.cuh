@@ -60,8 +60,11 @@
 #define FS_BLOCK (FS_MBLOCK * FS_MX)
 #define FS_CTPW (FS_TPW * (FS_MX - FS_PIPE))  // correlator threads per walker
 #if FS_PIPE
-#define FS_LPT 4                             // lags 4 lt .. 4 lt + 3
-#define FS_LAG(j) (4 * lt + (j))
+#ifndef FS_PLAGS
+#define FS_PLAGS 4
+#endif
+#define FS_LPT FS_PLAGS                      // consecutive lags of a helper lane, 4 or 2
+#define FS_LAG(j) (FS_LPT * lt + (j))
 #else
 #define FS_LPT ((FS_HALF_N + FS_CTPW - 1) / FS_CTPW)  // correlator lags owned per thread
 #define FS_LAG(j) (lt + (j) * FS_CTPW)
@@ -69,7 +72,7 @@
 #if FS_MX > 1 && (!FS_PARALLEL || FS_TPW > 32 || FS_GLOBAL || FS_NCOR == 0 || FS_NWALKERS % FS_WPB != 0)
 #error "correlator helpers need parallel-path walkers of at most 32 threads in shared memory, correlators, and full CTAs"
 #endif
-#if FS_PIPE && (FS_MX < 2 || FS_MBLOCK % 32 != 0 || FS_LEARNED || FS_SNSTRIDE < FS_DOF * (FS_N + (FS_N >> FS_S)) || FS_SNSTRIDE % 16 != 0 || FS_N % 8 != 0 || FS_CTPW < FS_N / 8)
+#if FS_PIPE && (FS_MX < 2 || FS_MBLOCK % 32 != 0 || FS_LEARNED || FS_SNSTRIDE < FS_DOF * (FS_N + (FS_N >> FS_S)) || FS_SNSTRIDE % 16 != 0 || FS_N % 8 != 0 || FS_CTPW < FS_HALF_N / FS_LPT)
 #error "pipelined correlator helpers need helper groups, whole warps of movers and a path snapshot"
 #endif
 #define FS_COR_REGS (FS_ACCUM != 3 && FS_LPT * FS_NCOR <= 16)
@@ -887,10 +890,10 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
     const int gl = FS_G > 1 ? tid_b % FS_G : 0;    // lane of the segment thread
     const bool mover = FS_MX == 1 || grp == 0;
     const bool owner = mover && gl == 0;           // writes the work-item's state back
-    // this thread's lags FS_LAG(j): lt + j * FS_CTPW; with FS_PIPE the helper lanes lt < N/8
-    // own lags 4 lt + j
+    // this thread's lags FS_LAG(j): lt + j * FS_CTPW; with FS_PIPE the helper lanes
+    // lt < N / (2 FS_LPT) own lags FS_LPT lt + j
     const int lt = (grp - FS_PIPE) * FS_TPW + t;
-    const bool lagger = FS_PIPE ? !mover && lt < FS_N / 8 : true;
+    const bool lagger = FS_PIPE ? !mover && lt < FS_HALF_N / FS_LPT : true;
     const int w0 = (blockIdx.x + a.block_offset) * FS_WPB;
     const int w = w0 + wl;
     const int n_here = min(FS_WPB, FS_NWALKERS - w0);
@@ -1315,14 +1318,53 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
             }
         };
 #else
-        // pipelined helpers: helper lane lt < N/8 sums lags 4 lt .. 4 lt + 3 of one
-        // measurement with the same four chains per lag (slices s1 mod 4, in slice order) and
-        // the same pairwise combination as the lag sums above, so the same bits; the slice
-        // values s1..s1+3 and the window s1 + 4 lt .. s1 + 4 lt + 7 come in 16-byte loads (2
-        // per 16 products), the window's upper half carried to the next step.  Reads stop at
-        // slice 4 lt + N + 3 < 3N/2 of the doubled values.
-        auto fs_cor_lags4 = [&](const FT *Cm) {
-            if (!(lt < FS_N / 8)) return;
+        // pipelined helpers: helper lane lt < N / (2 L) sums the L = FS_LPT lags L lt .. L lt + L - 1
+        // of one measurement with the same four chains per lag (slices s1 mod 4, in slice order)
+        // and the same pairwise combination as the lag sums above, so the same bits.
+        auto fs_cor_add = [&](int c, int j, const float (&p)[4]) {
+            const double m = fs_f2d(__fadd_rn(__fadd_rn(p[0], p[1]), __fadd_rn(p[2], p[3])));
+#if FS_COR_REGS
+            cacc[c][j] = __dadd_rn(cacc[c][j], m);
+#else
+            g_cor[c * FS_HALF_N + FS_LAG(j)] = __dadd_rn(g_cor[c * FS_HALF_N + FS_LAG(j)], m);
+#endif
+        };
+#if FS_LPT == 2
+        // 2 lags: the slice values s1..s1+3 in a 16-byte load, the next four of the window in two
+        // 8-byte ones (3 loads per 8 products); reads stop at slice 3N/2 + 3 <= 2N - 1
+        auto fs_cor_lags_pipe = [&](const FT *Cm) {
+            if (!lagger) return;
+#pragma unroll
+            for (int c = 0; c < FS_NCOR; c++) {
+                const float4 *cv4 = reinterpret_cast<const float4 *>(Cm + c * FS_CSTRIDE);
+                const float2 *wv2 = reinterpret_cast<const float2 *>(Cm + c * FS_CSTRIDE) + lt;
+                float pa[2][4], w[10];
+#pragma unroll
+                for (int k = 0; k < 4; k++) pa[0][k] = pa[1][k] = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 3; i++) *reinterpret_cast<float2 *>(w + 2 * i) = wv2[i];
+#pragma unroll 16
+                for (int q = 0; q < FS_N / 4; q++) {
+                    const float4 a4 = cv4[q];
+                    const float av[4] = {a4.x, a4.y, a4.z, a4.w};
+                    const float2 n0 = wv2[2 * q + 3], n1 = wv2[2 * q + 4];
+#pragma unroll
+                    for (int j = 0; j < 2; j++)
+#pragma unroll
+                        for (int k = 0; k < 4; k++) pa[j][k] = __fmaf_rn(av[k], w[k + j], pa[j][k]);
+                    w[0] = w[4]; w[1] = w[5];
+                    w[2] = n0.x; w[3] = n0.y; w[4] = n1.x; w[5] = n1.y;
+                }
+#pragma unroll
+                for (int j = 0; j < 2; j++) fs_cor_add(c, j, pa[j]);
+            }
+        };
+#else
+        // 4 lags: the slice values s1..s1+3 and the window's next four in 16-byte loads (2 per 16
+        // products), the window's upper half carried to the next step; reads stop at slice
+        // 4 lt + N + 3 < 3N/2 of the doubled values
+        auto fs_cor_lags_pipe = [&](const FT *Cm) {
+            if (!lagger) return;
 #pragma unroll
             for (int c = 0; c < FS_NCOR; c++) {
                 const float4 *cv4 = reinterpret_cast<const float4 *>(Cm + c * FS_CSTRIDE);
@@ -1346,17 +1388,10 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
                     w0 = w1;
                 }
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const double m =
-                        fs_f2d(__fadd_rn(__fadd_rn(pa[j][0], pa[j][1]), __fadd_rn(pa[j][2], pa[j][3])));
-#if FS_COR_REGS
-                    cacc[c][j] = __dadd_rn(cacc[c][j], m);
-#else
-                    g_cor[c * FS_HALF_N + FS_LAG(j)] = __dadd_rn(g_cor[c * FS_HALF_N + FS_LAG(j)], m);
-#endif
-                }
+                for (int j = 0; j < 4; j++) fs_cor_add(c, j, pa[j]);
             }
         };
+#endif
 #endif
 #endif
 
@@ -1377,7 +1412,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
                     fs_cor_put(x, s);
                 }
                 asm volatile("bar.sync 2, %0;" ::"n"(FS_BLOCK - FS_MBLOCK) : "memory");
-                fs_cor_lags4(C);
+                fs_cor_lags_pipe(C);
             }
         } else
 #endif
