@@ -69,7 +69,11 @@
 #define FS_LPT ((FS_HALF_N + FS_CTPW - 1) / FS_CTPW)  // correlator lags owned per thread
 #define FS_LAG(j) (lt + (j) * FS_CTPW)
 #endif
-#if FS_MX > 1 && (!FS_PARALLEL || FS_TPW > 32 || FS_GLOBAL || FS_NCOR == 0 || FS_NWALKERS % FS_WPB != 0)
+// Helpers and movers share CTA barriers, so every thread of a CTA has to run.  Where the walkers do
+// not fill the last CTA (FS_RAGGED, pipelined helpers only), its spare threads run on a path of
+// zeros and the last walker's generator rows, and write nothing to device memory.
+#define FS_RAGGED (FS_PIPE && FS_NWALKERS % FS_WPB != 0)
+#if FS_MX > 1 && (!FS_PARALLEL || FS_TPW > 32 || FS_GLOBAL || FS_NCOR == 0 || (FS_NWALKERS % FS_WPB != 0 && !FS_RAGGED))
 #error "correlator helpers need parallel-path walkers of at most 32 threads in shared memory, correlators, and full CTAs"
 #endif
 #if FS_PIPE && (FS_MX < 2 || FS_MBLOCK % 32 != 0 || FS_LEARNED || FS_SNSTRIDE < FS_DOF * (FS_N + (FS_N >> FS_S)) || FS_SNSTRIDE % 16 != 0 || FS_N % 8 != 0 || FS_CTPW < FS_HALF_N / FS_LPT)
@@ -91,6 +95,9 @@
 // wrap.
 #ifndef FS_PARTIALS
 #define FS_PARTIALS 0
+#endif
+#if FS_RAGGED && !FS_COR_REGS
+#error "a ragged last CTA needs its lag sums in registers"
 #endif
 #define FS_COR_FMA ((FS_ACCUM == 1 || FS_ACCUM == 2) && !FS_DOUBLE && FS_PARTIALS == 0)
 // Operator FP64 sums of FP32 builds ("fp64" accumulation, FS_PARTIALS 0, parallel-path
@@ -889,15 +896,15 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
     const int t = tid_b % FS_LPW / FS_G;
     const int gl = FS_G > 1 ? tid_b % FS_G : 0;    // lane of the segment thread
     const bool mover = FS_MX == 1 || grp == 0;
-    const bool owner = mover && gl == 0;           // writes the work-item's state back
     // this thread's lags FS_LAG(j): lt + j * FS_CTPW; with FS_PIPE the helper lanes
     // lt < N / (2 FS_LPT) own lags FS_LPT lt + j
     const int lt = (grp - FS_PIPE) * FS_TPW + t;
     const bool lagger = FS_PIPE ? !mover && lt < FS_HALF_N / FS_LPT : true;
     const int w0 = (blockIdx.x + a.block_offset) * FS_WPB;
-    const int w = w0 + wl;
     const int n_here = min(FS_WPB, FS_NWALKERS - w0);
     const bool active = wl < n_here;
+    const bool owner = mover && gl == 0 && active;  // writes the work-item's state back
+    const int w = FS_RAGGED && !active ? FS_NWALKERS - 1 : w0 + wl;
 
     // ---- path in (coalesced global reads; padded shared layout) ----
     {
@@ -924,13 +931,16 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
         }
 #endif
 #endif
+#if FS_RAGGED
+        for (int i = n_here * FS_WSTRIDE + tid_b; i < FS_WPB * FS_WSTRIDE; i += FS_BLOCK) s_path[i] = (FT)0;
+#endif
 #if FS_NHIST > 0
         for (int i = tid_b; i < FS_HBINS; i += FS_BLOCK) s_hist[i] = 0u;
 #endif
     }
     __syncthreads();
 
-    if (active) {
+    if (active || FS_RAGGED) {
 #if FS_PIPE
         // the movers' own barrier (whole warps; the helpers never wait on it)
 #if FS_MBLOCK == 32
@@ -970,7 +980,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
         // The walker's offset stream: every reference work-item of the walker advances an
         // identical copy; here one lane advances it in shared memory for the walker.
         FsIStream &is = s_istream[wl];
-        if (owner && t == 0) {
+        if (mover && gl == 0 && t == 0) {
 #if FS_COMPAT
             fs_rl_load<FS_NSKIP>(is.st, a.gtab + (size_t)tid * 28);
 #else
@@ -1444,7 +1454,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #if FS_OFF_PRE
                 const fs_u32 off = s_offs[wl][run * FS_MSTEPS + step];
 #else
-                if (owner && t == 0) s_off[wl] = fs_offset(is, FS_PARALLEL ? FS_SEG : FS_N);
+                if (mover && gl == 0 && t == 0) s_off[wl] = fs_offset(is, FS_PARALLEL ? FS_SEG : FS_N);
                 FS_WSYNC();
                 const fs_u32 off = s_off[wl];
 #endif
@@ -1504,6 +1514,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
             // counts of a slice's coordinates
             auto fs_count = [&](const FT *x) {
                 (void)x;
+                if (FS_RAGGED && !active) return;
 #if FS_BINS
                 {
                     int ok = 1, inc = 1, bi = 0;
@@ -1616,7 +1627,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #pragma unroll
             for (int j = 0; j < FS_LPT; j++) {
                 const int tau = FS_LAG(j);
-                if (lagger && tau < FS_HALF_N) g_cor[c * FS_HALF_N + tau] = cacc[c][j];
+                if (lagger && active && tau < FS_HALF_N) g_cor[c * FS_HALF_N + tau] = cacc[c][j];
             }
 #endif
 #if FS_GLOBAL

@@ -1,5 +1,5 @@
-"""Pipelined correlator helpers of two lags a lane against one walker per CTA (helpers after the
-moves, or none), and of the library's own choice for a run of few walkers: the same bits, IEEE
+"""Pipelined correlator helpers of two lags a lane, and with walkers that leave the last CTA
+ragged, against one walker per CTA (helpers after the moves, or none): the same bits, IEEE
 builds."""
 import types
 
@@ -18,7 +18,9 @@ def _gpu():
 
 @pytest.mark.parametrize("N,S,W,accumulation", [(16, 1, 12, "fp64"), (16, 2, 16, "kahan"), (32, 2, 20, "fp64"),
                                                 (64, 2, 6, "fp64"), (64, 1, 3, "fp64"), (128, 3, 40, "fp64"),
-                                                (128, 3, 2, "kahan"), (64, 3, 8, "fp64")])
+                                                (128, 3, 2, "kahan"), (64, 3, 8, "fp64"),
+                                                (128, 3, 41, "fp64"), (32, 2, 5, "fp64"), (64, 4, 9, "kahan"),
+                                                (16, 3, 1, "fp64"), (64, 2, 333, "fp64")])
 def test_two_lags_bit_identical(N, S, W, accumulation):
     kernel, kernel_args = engine()
     system = types.SimpleNamespace(DOF=1, potential="0.5 * x1 * x1", userCode="")
@@ -30,10 +32,12 @@ def test_two_lags_bit_identical(N, S, W, accumulation):
             enableBisection=True, enablePathShift=False, enableSingleNodeMove=False, enableBins=False,
             nbrOfWalkersPerWorkGroup=1, enableParallelizePath=True, enableGlobalPath=False, enableGlobalOldPath=False,
             operators=("x1 * x1",), correlators=("x1", "x1 * x1"), operatorRuns=3, metroStepsPerOperatorRun=2,
-            accumulation=accumulation, fastMath=False, walkersPerBlock=wpb, seed=S))
+            accumulation=accumulation, fastMath=False, walkersPerBlock=wpb, seed=S, histograms=("x1",),
+            histRange=(-2.0, 2.0), histBins=16))
         k.setPaths(p0)
         k.run(2)
-        got.append((k.getPaths(), k._raw_operators(), k.getAccepts(), k._raw_correlator()))
+        got.append((k.getPaths(), k._raw_operators(), k.getAccepts(), k._raw_correlator(), k.getSeeds(), k.getWalkerSeeds(),
+                    k.getHistogram(density=False)[1]))
         k.close()
     for a, b in zip(*got):
         assert np.array_equal(a, b)
