@@ -69,6 +69,7 @@ struct fs_handle {
     int tpw = 1, seg = 1, wpb = 1, block = 1, grid = 1;
     int lanes = 1;  // lanes that share a segment thread (FS_G)
     int cor_ilv = 0;  // correlator lags summed in one slice pass over a doubled slice buffer
+    int consec = 0;   // lags in consecutive fours without pipelined helpers (FS_CONSEC)
     int plags = 4;    // lags a pipelined helper lane sums (FS_PLAGS)
     int pipe = 0;     // correlator helpers one measurement behind the movers (FS_PIPE)
     long long snstride = 0;  // FS_PIPE: one path snapshot in shared memory, elements
@@ -340,7 +341,7 @@ static std::string gen_source(const fs_handle &h, const std::string &potential,
       << "\n#define FS_VCACHE " << (h.vstride || h.vglobal ? 1 : 0) << "\n#define FS_VSTRIDE " << h.vstride
       << "\n#define FS_VGLOBAL " << h.vglobal
       << "\n#define FS_COR_ILV " << h.cor_ilv << "\n#define FS_CWSTRIDE " << h.cwstride << "\n#define FS_MX "
-      << h.mx << "\n#define FS_PIPE " << h.pipe << "\n#define FS_PLAGS " << h.plags << "\n#define FS_SNSTRIDE " << h.snstride << "\n#define FS_G " << h.lanes << "\n";
+      << h.mx << "\n#define FS_PIPE " << h.pipe << "\n#define FS_PLAGS " << h.plags << "\n#define FS_CONSEC " << h.consec << "\n#define FS_SNSTRIDE " << h.snstride << "\n#define FS_G " << h.lanes << "\n";
     {
         const int mv = c.moves ? c.moves : FS_MOVE_BISECTION;
         const double nb = (double)c.n_slices / c.beta;
@@ -829,7 +830,16 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
             if (c.walkers_per_block > 0 && c.n_walkers % c.walkers_per_block) h->mx = 1, h->pipe = 0;
         }
         const long long lag_tpw = (long long)h->tpw * (h->mx - h->pipe);
-        const long long lpt = h->pipe ? h->plags : (c.n_slices / 2 + lag_tpw - 1) / lag_tpw;
+        // consecutive lags with wide loads where N/8 threads are there for them, although others then
+        // idle: four lags a thread, or two where four would leave a walker of at most 64 threads
+        // three quarters idle.  Us a run of 40 measurements, lags apart / four / two: N = 512, S = 3,
+        // 1000 walkers 753 / 315 / -; N = 2048, S = 3, 500 walkers 5850 / 2226 / -; N = 128, S = 1, 4000
+        // walkers 279 / 292 / 204; N = 1024, S = 1, 100 walkers 534 / 198 / 294.
+        h->consec = !h->pipe && !h->cors.empty() && c.enable_parallelize_path && !c.enable_double &&
+                    (c.accum == FS_ACCUM_FP64 || c.accum == FS_ACCUM_KAHAN) && c.partials == FS_PARTIALS_FP32 &&
+                    c.n_slices % 8 == 0 && lag_tpw >= c.n_slices / 8;
+        if (h->consec) h->plags = lag_tpw > c.n_slices / 4 && lag_tpw <= 64 ? 2 : 4;
+        const long long lpt = h->consec || h->pipe ? h->plags : (c.n_slices / 2 + lag_tpw - 1) / lag_tpw;
         h->cor_ilv = (c.accum != 0 && !c.enable_double && lpt <= 4) ? 1 : 0;
         // per-walker stride an odd multiple of 64 bytes: two walkers sharing a warp read
         // opposite bank halves

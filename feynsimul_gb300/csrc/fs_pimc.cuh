@@ -23,6 +23,9 @@
 
 #define FS_HALF_N (FS_N / 2)
 #define FS_THREADS (FS_NWALKERS * FS_TPW)
+// Lags in order (FS_CONSEC, set by the host where a walker has the N / 8 threads for it): a thread
+// sums 4 consecutive lags with two 16-byte loads per 16 products, like the pipelined helpers,
+// instead of lags FS_CTPW apart with a load a product.
 // Correlator helpers (FS_MX > 1, set by the host for correlator runs whose walkers have few
 // segment threads): the CTA holds FS_MX groups of FS_WPB x FS_TPW threads.  Group 0 runs the
 // moves and the per-slice measurement; every group sums correlator lags, so a walker's N/2
@@ -59,10 +62,13 @@
 #define FS_MBLOCK (FS_WPB * FS_LPW)          // threads that run the moves
 #define FS_BLOCK (FS_MBLOCK * FS_MX)
 #define FS_CTPW (FS_TPW * (FS_MX - FS_PIPE))  // correlator threads per walker
-#if FS_PIPE
 #ifndef FS_PLAGS
 #define FS_PLAGS 4
 #endif
+#ifndef FS_CONSEC
+#define FS_CONSEC 0
+#endif
+#if FS_PIPE || FS_CONSEC
 #define FS_LPT FS_PLAGS                      // consecutive lags of a helper lane, 4 or 2
 #define FS_LAG(j) (FS_LPT * lt + (j))
 #else
@@ -109,11 +115,11 @@
 #ifndef FS_COR_ILV
 #define FS_COR_ILV 0
 #endif
-#if FS_COR_ILV && !((FS_COR_FF || FS_COR_FMA) && FS_LPT <= 4 && (FS_PIPE || FS_LPT * FS_CTPW <= FS_N))
+#if FS_COR_ILV && !((FS_COR_FF || FS_COR_FMA) && FS_LPT <= 4 && (FS_PIPE || FS_CONSEC || FS_LPT * FS_CTPW <= FS_N))
 #error "FS_COR_ILV needs FP32 correlator partials and at most 4 lags per thread"
 #endif
-#if FS_PIPE && !(FS_COR_FMA && FS_COR_ILV)
-#error "pipelined correlator helpers sum FP32 partials over doubled slice values"
+#if (FS_PIPE || FS_CONSEC) && !(FS_COR_FMA && FS_COR_ILV)
+#error "consecutive lags need FP32 partials over doubled slice values"
 #endif
 // Slices whose coordinates a measurement loads at once: with one or two degrees of freedom a
 // slice's operator is a few instructions, and slice by slice the loop waits for each load
@@ -899,7 +905,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
     // this thread's lags FS_LAG(j): lt + j * FS_CTPW; with FS_PIPE the helper lanes
     // lt < N / (2 FS_LPT) own lags FS_LPT lt + j
     const int lt = (grp - FS_PIPE) * FS_TPW + t;
-    const bool lagger = FS_PIPE ? !mover && lt < FS_HALF_N / FS_LPT : true;
+    const bool lagger = FS_PIPE ? !mover && lt < FS_HALF_N / FS_LPT : FS_CONSEC ? lt < FS_HALF_N / FS_LPT : true;
     const int w0 = (blockIdx.x + a.block_offset) * FS_WPB;
     const int n_here = min(FS_WPB, FS_NWALKERS - w0);
     const bool active = wl < n_here;
@@ -1100,7 +1106,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #endif
             }
         };
-#if !FS_PIPE
+#if !FS_PIPE && !FS_CONSEC
         // one measurement's lag sums of the slice values in Cm, added to the lags this thread
         // owns: tau = lt + j * FS_CTPW
         auto fs_cor_lags = [&](const FT *Cm) {
@@ -1328,7 +1334,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
             }
         };
 #else
-        // pipelined helpers: helper lane lt < N / (2 L) sums the L = FS_LPT lags L lt .. L lt + L - 1
+        // consecutive lags (FS_CONSEC, and the pipelined helpers): lane lt < N / (2 L) sums the L = FS_LPT lags L lt .. L lt + L - 1
         // of one measurement with the same four chains per lag (slices s1 mod 4, in slice order)
         // and the same pairwise combination as the lag sums above, so the same bits.
         auto fs_cor_add = [&](int c, int j, const float (&p)[4]) {
@@ -1342,7 +1348,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
 #if FS_LPT == 2
         // 2 lags: the slice values s1..s1+3 in a 16-byte load, the next four of the window in two
         // 8-byte ones (3 loads per 8 products); reads stop at slice 3N/2 + 3 <= 2N - 1
-        auto fs_cor_lags_pipe = [&](const FT *Cm) {
+        auto fs_cor_lags = [&](const FT *Cm) {
             if (!lagger) return;
 #pragma unroll
             for (int c = 0; c < FS_NCOR; c++) {
@@ -1373,7 +1379,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
         // 4 lags: the slice values s1..s1+3 and the window's next four in 16-byte loads (2 per 16
         // products), the window's upper half carried to the next step; reads stop at slice
         // 4 lt + N + 3 < 3N/2 of the doubled values
-        auto fs_cor_lags_pipe = [&](const FT *Cm) {
+        auto fs_cor_lags = [&](const FT *Cm) {
             if (!lagger) return;
 #pragma unroll
             for (int c = 0; c < FS_NCOR; c++) {
@@ -1422,7 +1428,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
                     fs_cor_put(x, s);
                 }
                 asm volatile("bar.sync 2, %0;" ::"n"(FS_BLOCK - FS_MBLOCK) : "memory");
-                fs_cor_lags_pipe(C);
+                fs_cor_lags(C);
             }
         } else
 #endif
