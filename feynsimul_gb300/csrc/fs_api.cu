@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
+#include <map>
 #include <mutex>
 #include <sstream>
 #include <string>
@@ -59,6 +60,54 @@ struct FsCorStudyHost {
     float f, ks, kc, pad;
 };
 static_assert(sizeof(FsCorStudyHost) == 24, "study accumulator layout");
+
+// ------------------------------------------------------------------ page-locked host blocks
+// Page-locking memory takes 0.4 ms a block, an eighth of creating a small handle, so blocks of
+// destroyed handles and batches are kept for later ones: powers of two from 4 KB to 4 MB, at most
+// 8 MB idle in the process (a block beyond that is freed).  A block comes back only after its
+// owner's streams have drained.  Mapped and portable, so any device of the process may get it.
+static std::mutex g_pinned_mu;
+static auto &g_pinned_idle = *new std::multimap<size_t, void *>;  // by size; outlives every handle
+static size_t g_pinned_bytes = 0;                                 // in g_pinned_idle
+
+__attribute__((visibility("hidden"))) void *fsi_pinned_get(size_t bytes, size_t *size)
+{
+    size_t n = 4096;
+    while (n < bytes) n *= 2;
+    *size = n;
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        auto it = g_pinned_idle.find(n);
+        if (it != g_pinned_idle.end()) {
+            void *p = it->second;
+            g_pinned_idle.erase(it);
+            g_pinned_bytes -= n;
+            memset(p, 0, bytes);
+            return p;
+        }
+    }
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, n, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    memset(p, 0, bytes);
+    return p;
+}
+
+__attribute__((visibility("hidden"))) void fsi_pinned_put(void *p, size_t size)
+{
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        if (g_pinned_bytes + size <= (size_t)8 << 20) {
+            g_pinned_idle.emplace(size, p);
+            g_pinned_bytes += size;
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
 
 struct fs_handle {
     fs_config cfg{};
@@ -109,6 +158,7 @@ struct fs_handle {
     // raised one), and where they fit the accepts, the per-walker operator means and the
     // correlator moments
     void *pinned = nullptr;
+    size_t pinned_size = 0;
     int *status = nullptr;
     uint32_t *h_accepts = nullptr;
     double *h_wops = nullptr, *h_red = nullptr;
@@ -703,7 +753,7 @@ static void free_buffers(fs_handle *h)
                     h->d_mlp_frag, h->d_mlp_bias, h->d_red, h->d_shift_old, h->d_wops, h->d_vcache};
     for (void *p : bufs)
         if (p && p != h->h_accepts) cudaFree(p);
-    if (h->pinned) cudaFreeHost(h->pinned);
+    fsi_pinned_put(h->pinned, h->pinned_size);
 }
 
 // Results a run loop reads after every launch are small, and a device-to-host copy with its
@@ -716,14 +766,9 @@ static int host_results(fs_handle *h, size_t accepts, size_t wops, size_t red)
 {
     auto part = [](size_t bytes) { return bytes <= kHostResult ? (bytes + 255) / 256 * 256 : 0; };
     const size_t bytes = 256 + part(accepts) + part(wops) + part(red);
-    cudaError_t e = cudaHostAlloc(&h->pinned, bytes, cudaHostAllocMapped);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        h->pinned = nullptr;
-        return fail(h, FS_ERR_OOM, "Unable to allocate page-locked host memory (%zu bytes: %s)", bytes,
-                    cudaGetErrorString(e));
-    }
-    memset(h->pinned, 0, bytes);
+    h->pinned = fsi_pinned_get(bytes, &h->pinned_size);
+    if (!h->pinned)
+        return fail(h, FS_ERR_OOM, "Unable to allocate page-locked host memory (%zu bytes)", bytes);
     char *at = (char *)h->pinned;
     h->status = (int *)at;
     at += 256;

@@ -23,6 +23,8 @@ std::string fsi_prelude(bool dbl);
 const char *fsi_rng_src();
 const char *fsi_batch_src();
 int fsi_nskip_for(int lux);
+void *fsi_pinned_get(size_t bytes, size_t *size);
+void fsi_pinned_put(void *p, size_t size);
 int fsi_compile(const std::string &src, bool fast, std::string *cubin, std::string *log);
 
 #define FS_BATCH_MAX_S 10
@@ -60,6 +62,7 @@ struct fs_batch {
     cudaGraphExec_t gexec = nullptr;
     void *d_desc = nullptr, *d_items = nullptr, *d_counter = nullptr, *d_old = nullptr;
     std::vector<void *> allocs;
+    size_t pinned_size = 0;
     void *pinned = nullptr;        // page-locked host memory the kernel writes accepts and sums to, or null
     std::atomic<bool> idle{true};  // nothing was queued since the stream last drained
     bool timed = false;
@@ -97,7 +100,7 @@ static void free_batch(fs_batch *b)
     if (b->gexec) cudaGraphExecDestroy(b->gexec);
     if (b->graph) cudaGraphDestroy(b->graph);
     for (void *p : b->allocs) cudaFree(p);
-    if (b->pinned) cudaFreeHost(b->pinned);
+    fsi_pinned_put(b->pinned, b->pinned_size);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->lib) cudaLibraryUnload(b->lib);
@@ -359,8 +362,8 @@ extern "C" int fs_batch_create(int32_t n_types, const int32_t *type_dof, const c
             bytes += round((size_t)s.n_walkers * std::max(n_ops, 1) * 8) +
                      round((size_t)s.n_walkers * (s.n_slices >> s.bisection_level) * 4);
         if (bytes <= ((size_t)4 << 20)) {
-            CT(cuda(cudaHostAlloc(&b->pinned, bytes, cudaHostAllocMapped), "cudaHostAlloc"));
-            memset(b->pinned, 0, bytes);
+            b->pinned = fsi_pinned_get(bytes, &b->pinned_size);
+            if (!b->pinned) CT(bfail(FS_ERR_OOM, "Unable to allocate page-locked host memory (%zu bytes)", bytes));
             host_at = (char *)b->pinned;
         }
     }
