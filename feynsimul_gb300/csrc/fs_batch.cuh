@@ -226,9 +226,8 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
                         // Box-Muller evaluated for every degree of freedom and replaced by 0
                         // where v == 0 (kernel.c:349-353): no branch, so the compiler interleaves
                         // the degrees of freedom
-                        auto node_x = [&](int d, float u, float v) {
-                            float rz = __fmul_rn(__fmul_rn(sig, sqrtf(__fmul_rn(-2.f, __logf(v)))),
-                                                 __sinf(__fmul_rn(6.28318548f, u)));
+                        auto node_x = [&](int d, float angle, float v) {
+                            float rz = __fmul_rn(__fmul_rn(sig, sqrtf(__fmul_rn(-2.f, __logf(v)))), __sinf(angle));
                             rz = v != 0.f ? rz : 0.f;
                             FSB_AT(P, d, m) = __fadd_rn(__fmul_rn(0.5f, __fadd_rn(FSB_AT(P, d, l), FSB_AT(P, d, r))), rz);
                         };
@@ -239,7 +238,9 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
                             float uv[12];
                             g.template next_k<12>(uv);
 #pragma unroll
-                            for (int d = 0; d < 6; d++) node_x(d0 + d, uv[2 * d], uv[2 * d + 1]);
+                            for (int d = 0; d < 6; d++)
+                                node_x(d0 + d, __fmul_rn(6.28318548f * FS_RL_UNIT, uv[2 * d]),
+                                       __fmul_rn(uv[2 * d + 1], FS_RL_UNIT));
                         }
 #pragma unroll 1
                         for (int d = DOF / 6 * 6; d < DOF; d++) {
@@ -249,7 +250,7 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
 #endif
                             const float u = fsb_uniform(g);
                             const float v = fsb_uniform(g);
-                            node_x(d, u, v);
+                            node_x(d, __fmul_rn(6.28318548f, u), v);
                         }
                     }
                 }

@@ -207,6 +207,9 @@
 #define FS_TWO_PI 6.28318548f  // 2 * float(pi), as the reference's single-precision constant
 #endif
 
+// 2 pi times a generator value in its own unit (fs_rng.cuh): the same product, one rounding
+#define FS_RAW_ANGLE (6.28318548f * FS_RL_UNIT)
+
 // ---------------------------------------------------------------- streams
 #if FS_RANLUX
 #if FS_DOUBLE
@@ -359,8 +362,8 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
             // bookkeeping and six independent log / sqrt / sin chains (5 atoms, N = 128, 4000 walkers:
             // 454 -> 377 us a run; 10 atoms, N = 256: 1137 -> 1021).  Not under a register budget of
             // 64, where the twelve values spill (10 atoms, N = 1024 in device memory: 3830 against 3920)
-            auto node_x = [&](int d, float u, float v) {
-                float rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(FS_MUL((FT)FS_TWO_PI, u)));
+            auto node_x = [&](int d, float angle, float v) {
+                float rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(angle));
                 rz = v != 0.0f ? rz : 0.0f;
                 FS_AT(P, d, m) = FS_ADD(FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r))), rz);
             };
@@ -369,13 +372,14 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
                 float uv[12];
                 g.template next_k<12>(uv);
 #pragma unroll
-                for (int d = 0; d < 6; d++) node_x(d0 + d, uv[2 * d], uv[2 * d + 1]);
+                for (int d = 0; d < 6; d++)
+                    node_x(d0 + d, FS_MUL(FS_RAW_ANGLE, uv[2 * d]), FS_MUL(uv[2 * d + 1], FS_RL_UNIT));
             }
 #pragma unroll 1
             for (int d = FS_DOF / 6 * 6; d < FS_DOF; d++) {
                 const float u = fs_uniform(g);
                 const float v = fs_uniform(g);
-                node_x(d, u, v);
+                node_x(d, FS_MUL((FT)FS_TWO_PI, u), v);
             }
 #else
 #if FS_RANLUX && !FS_DOUBLE && (2 * FS_DOF) % 4 == 0
@@ -384,18 +388,18 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
             g.template next_k<2 * FS_DOF>(uv);
 #pragma unroll
             for (int d = 0; d < FS_DOF; d++) {
-                const FT u = uv[2 * d];
-                const FT v = uv[2 * d + 1];
+                const FT angle = FS_MUL(FS_RAW_ANGLE, uv[2 * d]);
+                const FT v = FS_MUL(uv[2 * d + 1], FS_RL_UNIT);
 #else
             FS_DOF_UNROLL
             for (int d = 0; d < FS_DOF; d++) {
-                const FT u = fs_uniform(g);
+                const FT angle = FS_MUL((FT)FS_TWO_PI, fs_uniform(g));
                 const FT v = fs_uniform(g);
 #endif
 #if FS_LEARNED
                 if (n == 1) {
                     FT z = (FT)0;
-                    if (v != (FT)0) z = FS_MUL(FS_SQRT(FS_MUL((FT)-2, FS_LOG(v))), FS_SIN(FS_MUL((FT)FS_TWO_PI, u)));
+                    if (v != (FT)0) z = FS_MUL(FS_SQRT(FS_MUL((FT)-2, FS_LOG(v))), FS_SIN(angle));
                     const FT mid = FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r)));
                     const FT xo = FS_AT(P, d, m);
                     const FT xn = lmu[d] + lsd[d] * z;
@@ -409,8 +413,7 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
                 // for v == 0 (kernel.c:349-351).  Evaluated unconditionally and selected: log 0
                 // is -inf, so that lane's product is infinite or NaN and is discarded, and no
                 // branch is taken per degree of freedom.
-                FT rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))),
-                               FS_SIN(FS_MUL((FT)FS_TWO_PI, u)));
+                FT rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(angle));
                 rz = v != (FT)0 ? rz : (FT)0;
                 FS_AT(P, d, m) = FS_ADD(FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r))), rz);
             }
@@ -540,7 +543,8 @@ __device__ __forceinline__ int fs_bisect_lanes(FT *P, FT *Vc, fs_u32 start, FsUS
                 for (int j = 0; j < FS_G; j++) {
                     if (FS_DOF % FS_G != 0 && k * FS_G + j >= FS_DOF) break;
 #if FS_RANLUX && !FS_DOUBLE
-                    const FT uj = uv[2 * (k * FS_G + j)], vj = uv[2 * (k * FS_G + j) + 1];
+                    const FT uj = uv[2 * (k * FS_G + j)];
+                    const FT vj = FS_MUL(uv[2 * (k * FS_G + j) + 1], FS_RL_UNIT);
 #else
                     const FT uj = fs_uniform(g);
                     const FT vj = fs_uniform(g);
@@ -549,7 +553,12 @@ __device__ __forceinline__ int fs_bisect_lanes(FT *P, FT *Vc, fs_u32 start, FsUS
                     v = j == gl ? vj : v;
                 }
                 const int d = k * FS_G + gl;
-                FT rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(FS_MUL((FT)FS_TWO_PI, u)));
+#if FS_RANLUX && !FS_DOUBLE
+                const FT angle = FS_MUL(FS_RAW_ANGLE, u);
+#else
+                const FT angle = FS_MUL((FT)FS_TWO_PI, u);
+#endif
+                FT rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(angle));
                 rz = v != (FT)0 ? rz : (FT)0;
                 if (FS_DOF % FS_G == 0 || d < FS_DOF)
                     FS_AT(P, d, m) = FS_ADD(FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r))), rz);
@@ -1726,7 +1735,8 @@ extern "C" __global__ void fs_ranlux_dump(const fs_u64 *xs, int n, int n_calls, 
         float o0, o1, o2, o3;
         fs_rl_next4<FS_NSKIP>(r, o0, o1, o2, o3);
         float *o = out + ((size_t)i * n_calls + c) * 4;
-        o[0] = o0; o[1] = o1; o[2] = o2; o[3] = o3;
+        o[0] = __fmul_rn(o0, FS_RL_UNIT); o[1] = __fmul_rn(o1, FS_RL_UNIT);
+        o[2] = __fmul_rn(o2, FS_RL_UNIT); o[3] = __fmul_rn(o3, FS_RL_UNIT);
     }
     fs_rl_store_new<FS_NSKIP>(r, states + (size_t)i * 28);
 }

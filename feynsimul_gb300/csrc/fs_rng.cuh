@@ -253,6 +253,11 @@ __device__ __forceinline__ fs_u32 fs_rl_digit8(const FsRanlux &r)
     return r.w[j + 2] & 0xFFFFFF00u;
 }
 
+// Generator values leave this part in units of 2^-32 (FS_RL_UNIT): the conversion of a digit
+// shifted left by 8, without the multiplication.  A power of two commutes with every rounding
+// here (no value is below 2^-48), so a user that multiplies anyway folds it in.
+#define FS_RL_UNIT 0x1p-32f
+
 // output of the step that updated digit P (pyopencl-ranluxcl.cl:363-378): a value below 2^-12
 // gets the bits of the digit nine steps before, zero becomes 2^-48.  That digit is as it was
 // at the step until a skip or the step of its own position in the next cycle.
@@ -260,40 +265,50 @@ template <int P>
 __device__ __forceinline__ float fs_rl_value(const FsRanlux &r)
 {
     const fs_u32 v = fs_rl_digit8<P>(r);
-    const float hi = __fmul_rn(__uint2float_rn(v), 0x1p-32f);
-    const float lo = __fmul_rn(__uint2float_rn(fs_rl_digit8<(P + 15) % 24>(r)), 0x1p-56f);
+    const float hi = __uint2float_rn(v);
+    const float lo = __fmul_rn(__uint2float_rn(fs_rl_digit8<(P + 15) % 24>(r)), 0x1p-24f);
     float out = v < (4096u << 8) ? __fadd_rn(hi, lo) : hi;
-    return out == 0.0f ? 0x1p-48f : out;
+    return out == 0.0f ? 0x1p-16f : out;
 }
 
-// The four outputs of quad Q, whose chain has run: the plain conversion, and the small-value
-// correction of fs_rl_value only when some lane of the warp drew a value below 2^-12
-// (probability 2^-12 per value).
+// plain conversions of quad Q, whose chain has run, and the smallest of its digits
 template <int Q>
-__device__ __forceinline__ void fs_rl_out4(const FsRanlux &r, float *o)
+__device__ __forceinline__ fs_u32 fs_rl_plain4(const FsRanlux &r, float *o)
 {
     const fs_u32 d0 = fs_rl_digit8<4 * Q>(r), d1 = fs_rl_digit8<4 * Q + 1>(r);
     const fs_u32 d2 = fs_rl_digit8<4 * Q + 2>(r), d3 = fs_rl_digit8<4 * Q + 3>(r);
-    o[0] = __fmul_rn(__uint2float_rn(d0), 0x1p-32f);
-    o[1] = __fmul_rn(__uint2float_rn(d1), 0x1p-32f);
-    o[2] = __fmul_rn(__uint2float_rn(d2), 0x1p-32f);
-    o[3] = __fmul_rn(__uint2float_rn(d3), 0x1p-32f);
-    if (__any_sync(__activemask(), min(min(d0, d1), min(d2, d3)) < (4096u << 8))) {
-        o[0] = fs_rl_value<4 * Q>(r);
-        o[1] = fs_rl_value<4 * Q + 1>(r);
-        o[2] = fs_rl_value<4 * Q + 2>(r);
-        o[3] = fs_rl_value<4 * Q + 3>(r);
-    }
+    o[0] = __uint2float_rn(d0);
+    o[1] = __uint2float_rn(d1);
+    o[2] = __uint2float_rn(d2);
+    o[3] = __uint2float_rn(d3);
+    return min(min(d0, d1), min(d2, d3));
 }
 
-// NQ quads starting at quad Q, their steps in one chain
+template <int Q>
+__device__ __forceinline__ void fs_rl_value4(const FsRanlux &r, float *o)
+{
+    o[0] = fs_rl_value<4 * Q>(r);
+    o[1] = fs_rl_value<4 * Q + 1>(r);
+    o[2] = fs_rl_value<4 * Q + 2>(r);
+    o[3] = fs_rl_value<4 * Q + 3>(r);
+}
+
+// NQ quads starting at quad Q, their steps in one chain: the plain conversions, and the
+// small-value correction of fs_rl_value only when some lane of the warp drew a value below 2^-12
+// (probability 2^-12 per value).  One vote for all of them, not one a quad: the trimer sweep went
+// from 5.53 to 5.21 ms a run, and to 5.11 with the values in units of 2^-32.
 template <int Q, int NQ>
 __device__ __forceinline__ void fs_rl_quads(FsRanlux &r, float *o)
 {
     fs_rl_chain<Q, NQ>(r);
-    fs_rl_out4<Q>(r, o);
-    if (NQ > 1) fs_rl_out4<(Q + 1) % 6>(r, o + 4);
-    if (NQ > 2) fs_rl_out4<(Q + 2) % 6>(r, o + 8);
+    fs_u32 least = fs_rl_plain4<Q>(r, o);
+    if (NQ > 1) least = min(least, fs_rl_plain4<(Q + 1) % 6>(r, o + 4));
+    if (NQ > 2) least = min(least, fs_rl_plain4<(Q + 2) % 6>(r, o + 8));
+    if (__any_sync(__activemask(), least < (4096u << 8))) {
+        fs_rl_value4<Q>(r, o);
+        if (NQ > 1) fs_rl_value4<(Q + 1) % 6>(r, o + 4);
+        if (NQ > 2) fs_rl_value4<(Q + 2) % 6>(r, o + 8);
+    }
 }
 
 // NSKIP steps from digit 0, and the frame moved to where they end
@@ -319,7 +334,7 @@ __device__ __forceinline__ void fs_rl_skip(FsRanlux &r)
     }
 }
 
-// four outputs (ranluxcl32), then the skip after every 24 outputs
+// four outputs (ranluxcl32, in units of 2^-32), then the skip after every 24 outputs
 template <int NSKIP>
 __device__ __forceinline__ void fs_rl_next4(FsRanlux &r, float &o0, float &o1, float &o2, float &o3)
 {
@@ -341,7 +356,7 @@ __device__ __forceinline__ void fs_rl_next4(FsRanlux &r, float &o0, float &o1, f
 
 // twelve outputs, the same as three calls of next4: straight-line code per starting quad, and
 // one copy of the skip (a loop over next4 spends four selects, a branch and eight moves a
-// quad; the trimer sweep took 5.96 ms with it and takes 5.57 ms)
+// quad; the trimer sweep took 5.96 ms with it and 5.57 ms so, before the single vote)
 template <int NSKIP>
 __device__ __forceinline__ void fs_rl_next12(FsRanlux &r, float (&c)[12])
 {
@@ -465,7 +480,7 @@ __device__ __forceinline__ void fs_rl_store_new(const FsRanlux &r, fs_u32 *t)
 template <int NSKIP>
 struct FsRanluxStream {
     FsRanlux st;
-    float b0, b1, b2, b3;
+    float b0, b1, b2, b3;  // in units of 2^-32
     fs_u32 count;
 
     __device__ __forceinline__ float next()
@@ -473,11 +488,11 @@ struct FsRanluxStream {
         fs_u32 c = count & 3u;
         if (c == 0u) fs_rl_next4<NSKIP>(st, b0, b1, b2, b3);
         count++;
-        return c == 0u ? b0 : (c == 1u ? b1 : (c == 2u ? b2 : b3));
+        return __fmul_rn(c == 0u ? b0 : (c == 1u ? b1 : (c == 2u ? b2 : b3)), FS_RL_UNIT);
     }
 
-    // K consecutive values (K a multiple of 4), the same values next() would return K
-    // times: the rem still-buffered values first, then K/4 fresh quadruples, the last rem
+    // K consecutive values (K a multiple of 4) in units of 2^-32, the same values next() would
+    // return K times: the rem still-buffered values first, then K/4 fresh quadruples, the last rem
     // of which stay buffered.  One branch per K values instead of one per value.
     template <int K>
     __device__ __forceinline__ void next_k(float (&u)[K])
@@ -546,6 +561,10 @@ struct FsRanluxStream64 {
     {
         float v0, v1, v2, v3;
         fs_rl_next4<NSKIP>(st, v0, v1, v2, v3);
+        v0 = __fmul_rn(v0, FS_RL_UNIT);
+        v1 = __fmul_rn(v1, FS_RL_UNIT);
+        v2 = __fmul_rn(v2, FS_RL_UNIT);
+        v3 = __fmul_rn(v3, FS_RL_UNIT);
         if (v0 == 0x1p-48f) v0 = 0.0f;
         if (v2 == 0x1p-48f) v2 = 0.0f;
         // v0 + v1 / 2^24, the exact quotient rounded into the sum: one FP64 operation where a
