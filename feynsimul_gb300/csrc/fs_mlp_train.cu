@@ -49,19 +49,21 @@ __device__ __forceinline__ fs_bf16 f2bf(float x)
 
 // ---------------------------------------------------------------- tcgen05 training
 // The same forward pass, loss and backward pass on the fifth-generation tensor cores, with
-// the same BF16 rounding points.  One CTA = 8 warps, persistent over 128-row tiles; a row of a
-// tile (a tensor-memory lane) belongs to two threads, r and r + 128, which take half of its
+// the same BF16 rounding points.  One CTA = 16 warps, persistent over 128-row tiles; a row of a
+// tile (a tensor-memory lane) belongs to the four threads r + 128 k, which take a quarter of its
 // columns each in every epilogue (a warp reads the 32 lanes of its number modulo 4).  The step is
-// a chain of 8 MMA groups with an epilogue between; of one tile's 34 thousand cycles (42 with one
-// warp a lane quarter and gradients stored line by line) the MMAs and their waits are about 7, the
-// epilogues 15, the weights 5 and the gradient's way out 5.  A step on 4096 rows, optimiser and
-// gather included, took 105 us in ten launches and takes 31 in three.
+// a chain of 8 MMA groups with an epilogue between.  With two threads a row, one tile took 34
+// thousand cycles (42 with one, and gradients stored line by line): the MMAs and their waits about
+// 7, the epilogues 15, the weights 5 and the gradient's way out 5.  So the epilogues have four
+// threads a row, and the weight-gradient MMAs, which nothing in the tile waits for, run behind the
+// next epilogue.  A step on 4096 rows, optimiser and gather included, took 105 us in ten launches;
+// 31 in three launches with two threads a row, and 27 now, the optimiser's launch overlapped too.
 // Rows of a training set are gathered in place by an index array.  Tensor memory (512 FP32
 // columns): the layer accumulator F (a forward layer's output or a hidden gradient dA), and
 // the weight gradients summed over the CTA's tiles: dW2 and dW3 (128 columns each), dW1 (16)
 // and dW4 transposed (16; its M is the 128 inputs).  Shared memory holds BF16 tiles in the
-// canonical layout of fs_tc.cuh: the activations a1..a3 and the hidden gradient g (128 x
-// 128, rows = the tile's rows), the input x and the output gradient dz4 (128 x 16), and the
+// canonical layout of fs_tc.cuh: the activations a1..a3 and the hidden gradient g (in turn g, a3
+// and g again, each 128 x 128, rows = the tile's rows), the input x and the output gradient dz4 (128 x 16), and the
 // weights W1..W4 ([out][in]).  The forward GEMMs read them K-major; dA = dZ W reads W
 // MN-major, and dW = dZ^T A reads dZ and A MN-major (K = the tile's rows), so no tile is
 // transposed.  The six 128-wide tiles come first and the allocation is padded, so every
@@ -71,7 +73,7 @@ __device__ __forceinline__ fs_bf16 f2bf(float x)
 // A CTA's gradient goes to its own row of `part` for the optimiser step to add up in order
 // (fs_mlp_train_batch: the same training run gives the same bits), or, without one, to grad
 // by atomics (fs_mlp_train_step).
-#define TT_THREADS 256
+#define TT_THREADS 512
 #define TT_TMEM_COLS 512
 #define TT_F 0u
 #define TT_DW2 128u
@@ -93,7 +95,7 @@ struct TtSmem {
     float bias[128 * 3 + 16];
     float db[4][128 * 3 + 16];  // bias gradients of each quarter of a tile's rows
     float loss[4];
-    alignas(8) unsigned long long mbar;
+    alignas(8) unsigned long long mbar, mbar_last;
     unsigned tmem_base;
     int give_up;
 };
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
     extern __shared__ __align__(1024) unsigned char tt_raw[];
     TtSmem &S = *reinterpret_cast<TtSmem *>(tt_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int r = tid & 127, half = tid >> 7;  // row of the tile, half of its columns
+    const int r = tid & 127, quarter = tid >> 7;  // row of the tile, quarter of its columns
     const int n_tiles = (n_rows + 127) / 128;
     const uint32_t mbar = tc_smem(&S.mbar);
 
@@ -143,15 +145,15 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
     const int row0 = (int)blockIdx.x * 128 + r;
     const bool valid0 = row0 < n_rows;
     size_t src = valid0 && pick ? (size_t)pick[row0] : (size_t)row0;
-    // half a row of x, and the row's z (the threads of half 0 use it)
+    // half a row of x (quarters 0 and 1), and the row's z (quarter 0)
     float4 xv[2], zv[2];
     auto fetch = [&](bool valid) {
-        const float4 *xr = reinterpret_cast<const float4 *>(xin + src * 16 + 8 * half);
+        const float4 *xr = reinterpret_cast<const float4 *>(xin + src * 16 + 8 * (quarter & 1));
 #pragma unroll
-        for (int c = 0; c < 2; c++) xv[c] = valid ? xr[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int c = 0; c < 2; c++) xv[c] = valid && quarter < 2 ? xr[c] : make_float4(0.f, 0.f, 0.f, 0.f);
         float *z = reinterpret_cast<float *>(zv);
 #pragma unroll
-        for (int d = 0; d < 8; d++) z[d] = valid && half == 0 && d < dof ? zin[src * 8 + d] : 0.f;
+        for (int d = 0; d < 8; d++) z[d] = valid && quarter == 0 && d < dof ? zin[src * 8 + d] : 0.f;
     };
     // ---- weights (the BF16 training copy, [out][in]) into canonical tiles, eight
     // consecutive inputs (one core-matrix row, 16 bytes) per load and store; a warp takes 8
@@ -169,8 +171,10 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
         tile128(S.w2, Q_W2, 128);
         tile128(S.w3, Q_W3, 128);
         tile128(S.w4, Q_W4, 16);
-        const int row = warp * 16 + (lane & 15), k = lane >> 4;  // 8 warps x 16 rows of 2 core matrices
-        *reinterpret_cast<uint4 *>(S.w1 + tc_off(row, k * 8, 16)) = q[Q_W1 / 8 + row * 2 + k];
+        if (warp < 8) {
+            const int row = warp * 16 + (lane & 15), k = lane >> 4;  // 16 rows of 2 core matrices a warp
+            *reinterpret_cast<uint4 *>(S.w1 + tc_off(row, k * 8, 16)) = q[Q_W1 / 8 + row * 2 + k];
+        }
     }
     fetch(valid0);
     for (int i = tid; i < 128; i += TT_THREADS) {
@@ -184,6 +188,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
     if (tid == 0) {
         S.give_up = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&S.mbar_last)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -202,9 +207,13 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
     bool ok = true, first = true;
     float *const db = S.db[warp & 3];
 
+    // the optimiser's CTAs may take their places now; they wait for this grid's end
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
     // one step: the operands made visible to the tensor cores, thread 0 issues the MMAs and
-    // commits, every thread waits (bounded) for them
-    auto step = [&](auto &&issue) {
+    // commits, every thread waits (bounded) for them.  The MMAs of `after` run behind them, during
+    // the epilogue: the next step's wait covers them.
+    auto step = [&](auto &&issue, auto &&after) {
         tc_fence_async();
         tc_fence_before();
         __syncthreads();
@@ -212,6 +221,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
         if (tid == 0) {
             issue();
             tc_commit(mbar);
+            after();
         }
         if (!tc_wait(mbar, phase)) S.give_up = 1;
         phase ^= 1u;
@@ -220,10 +230,11 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
         ok = S.give_up == 0;
         return ok;
     };
+    auto none = [] {};
     // forward epilogue: act = BF16(relu(F + b))
     auto relu_out = [&](fs_bf16 *act, const float *b) {
 #pragma unroll 1
-        for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 16) {
+        for (int c0 = 32 * quarter; c0 < 32 * quarter + 32; c0 += 16) {
             float v[16];
             tc_ld16(t_row + TT_F + (uint32_t)c0, v);
 #pragma unroll
@@ -233,9 +244,9 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
         }
     };
     // backward epilogue: dZ = F * (act > 0) -> g as BF16, its FP32 column sums into dbl
-    auto grad_out = [&](const fs_bf16 *act, float *dbl) {
-#pragma unroll 1
-        for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 32) {
+    auto grad_out = [&](const fs_bf16 *act, fs_bf16 *g, float *dbl) {
+        {
+            const int c0 = 32 * quarter;
             float v[32];
             tc_ld16(t_row + TT_F + (uint32_t)c0, *reinterpret_cast<float(*)[16]>(v));
             tc_ld16(t_row + TT_F + (uint32_t)c0 + 16u, *reinterpret_cast<float(*)[16]>(v + 16));
@@ -248,7 +259,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
                     if (!(__uint_as_float(w[e] << 16) > 0.f)) v[8 * q + 2 * e] = 0.f;
                     if (!(__uint_as_float(w[e] & 0xFFFF0000u) > 0.f)) v[8 * q + 2 * e + 1] = 0.f;
                 }
-                tc_st8(S.g + tc_off(r, c0 + 8 * q, 128), v + 8 * q);
+                tc_st8(g + tc_off(r, c0 + 8 * q, 128), v + 8 * q);
             }
             tt_colsum32(v, dbl + c0, lane, 32);
         }
@@ -261,33 +272,33 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
             src = valid && pick ? (size_t)pick[row] : (size_t)row;
             fetch(valid);
         }
-        tc_st8(S.x + tc_off(r, 8 * half, 16), reinterpret_cast<const float *>(xv));
+        if (quarter < 2) tc_st8(S.x + tc_off(r, 8 * quarter, 16), reinterpret_cast<const float *>(xv));
         // ---- forward ----
-        if (!step([&] { tc_mma(tmem + TT_F, tc_desc(S.x, 16), tc_desc(S.w1, 16), tc_idesc(128, 128), 0); }))
+        if (!step([&] { tc_mma(tmem + TT_F, tc_desc(S.x, 16), tc_desc(S.w1, 16), tc_idesc(128, 128), 0); }, none))
             break;
         relu_out(S.a1, S.bias);
         if (!step([&] {
                 for (int kk = 0; kk < 8; kk++)
                     tc_mma(tmem + TT_F, tc_desc(S.a1 + kk * 128, 128), tc_desc(S.w2 + kk * 128, 128),
                            tc_idesc(128, 128), kk > 0);
-            }))
+            }, none))
             break;
         relu_out(S.a2, S.bias + 128);
         if (!step([&] {
                 for (int kk = 0; kk < 8; kk++)
                     tc_mma(tmem + TT_F, tc_desc(S.a2 + kk * 128, 128), tc_desc(S.w3 + kk * 128, 128),
                            tc_idesc(128, 128), kk > 0);
-            }))
+            }, none))
             break;
         relu_out(S.a3, S.bias + 256);
         if (!step([&] {
                 for (int kk = 0; kk < 8; kk++)
                     tc_mma(tmem + TT_F, tc_desc(S.a3 + kk * 128, 128), tc_desc(S.w4 + kk * 128, 128),
                            tc_idesc(128, 16), kk > 0);
-            }))
+            }, none))
             break;
         // ---- loss and its gradient for this thread's row ----
-        if (half == 0) {
+        if (quarter == 0) {
             float z4[16], g[32];
             tc_ld16(t_row + TT_F, z4);
 #pragma unroll
@@ -324,46 +335,50 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
         }
         // ---- backward ----
         const uint32_t acc0 = first ? 0u : 1u;
-        if (!step([&] {
+        if (!step([&] {  // dA3 = dZ4 W4
+                tc_mma(tmem + TT_F, tc_desc(S.dz4, 16), tc_desc_mn(S.w4, 128), tc_idesc(128, 128, false, true), 0);
+            }, [&] {
                 for (int kk = 0; kk < 8; kk++)  // dW4^T += A3^T dZ4 (M = inputs, N = outputs)
                     tc_mma(tmem + TT_DW4, tc_desc_mn(S.a3 + kk * 2048, 128), tc_desc_mn(S.dz4 + kk * 256, 16),
                            tc_idesc(128, 16, true, true), acc0 | (kk > 0));
-                // dA3 = dZ4 W4
-                tc_mma(tmem + TT_F, tc_desc(S.dz4, 16), tc_desc_mn(S.w4, 128), tc_idesc(128, 128, false, true), 0);
             }))
             break;
-        grad_out(S.a3, db + 256);
+        grad_out(S.a3, S.g, db + 256);
         if (!step([&] {
-                for (int kk = 0; kk < 8; kk++)  // dW3 += dZ3^T A2
-                    tc_mma(tmem + TT_DW3, tc_desc_mn(S.g + kk * 2048, 128), tc_desc_mn(S.a2 + kk * 2048, 128),
-                           tc_idesc(128, 128, true, true), acc0 | (kk > 0));
                 for (int kk = 0; kk < 8; kk++)  // dA2 = dZ3 W3
                     tc_mma(tmem + TT_F, tc_desc(S.g + kk * 128, 128), tc_desc_mn(S.w3 + kk * 2048, 128),
                            tc_idesc(128, 128, false, true), kk > 0);
-            }))
-            break;
-        grad_out(S.a2, db + 128);
-        if (!step([&] {
-                for (int kk = 0; kk < 8; kk++)  // dW2 += dZ2^T A1
-                    tc_mma(tmem + TT_DW2, tc_desc_mn(S.g + kk * 2048, 128), tc_desc_mn(S.a1 + kk * 2048, 128),
+            }, [&] {
+                for (int kk = 0; kk < 8; kk++)  // dW3 += dZ3^T A2
+                    tc_mma(tmem + TT_DW3, tc_desc_mn(S.g + kk * 2048, 128), tc_desc_mn(S.a2 + kk * 2048, 128),
                            tc_idesc(128, 128, true, true), acc0 | (kk > 0));
-                for (int kk = 0; kk < 8; kk++)  // dA1 = dZ2 W2
-                    tc_mma(tmem + TT_F, tc_desc(S.g + kk * 128, 128), tc_desc_mn(S.w2 + kk * 2048, 128),
-                           tc_idesc(128, 128, false, true), kk > 0);
             }))
             break;
-        grad_out(S.a1, db);
+        // dW3 still reads g; a3 and its reader dW4 are done
+        grad_out(S.a2, S.a3, db + 128);
+        if (!step([&] {
+                for (int kk = 0; kk < 8; kk++)  // dA1 = dZ2 W2
+                    tc_mma(tmem + TT_F, tc_desc(S.a3 + kk * 128, 128), tc_desc_mn(S.w2 + kk * 2048, 128),
+                           tc_idesc(128, 128, false, true), kk > 0);
+            }, [&] {
+                for (int kk = 0; kk < 8; kk++)  // dW2 += dZ2^T A1
+                    tc_mma(tmem + TT_DW2, tc_desc_mn(S.a3 + kk * 2048, 128), tc_desc_mn(S.a1 + kk * 2048, 128),
+                           tc_idesc(128, 128, true, true), acc0 | (kk > 0));
+            }))
+            break;
+        grad_out(S.a1, S.g, db);
         if (!step([&] {
                 for (int kk = 0; kk < 8; kk++)  // dW1 += dZ1^T X
                     tc_mma(tmem + TT_DW1, tc_desc_mn(S.g + kk * 2048, 128), tc_desc_mn(S.x + kk * 256, 16),
                            tc_idesc(128, 16, true, true), acc0 | (kk > 0));
-            }))
+            }, none))
             break;
         first = false;
     }
     if (ok && !first) {
         // the CTA's weight gradients out of tensor memory: lane r is output row r of dW1..dW3 and
-        // input column r of dW4; the row's two threads take dW2, dW1 and dW3, dW4
+        // input column r of dW4; the row's four threads take half of dW2 or dW3 each, two of them
+        // dW1 and dW4 too
         // (16-byte vector atomics: the parameter offsets of W1..W3 are multiples of 4 floats)
         float *const out = part ? part + (size_t)blockIdx.x * TT_PART : grad;
         auto put4 = [&](float *dst, const float *v) {
@@ -375,19 +390,19 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
             if (part) *dst = v;
             else atomicAdd(dst, v);
         };
-        const uint32_t t_dw = t_row + (half == 0 ? TT_DW2 : TT_DW3);
-        const int p_w = half == 0 ? P_W2 : P_W3;
+        const uint32_t t_dw = t_row + (quarter < 2 ? TT_DW2 : TT_DW3);
+        const int p_w = quarter < 2 ? P_W2 : P_W3, first_c = 64 * (quarter & 1);
 #pragma unroll 2
-        for (int c0 = 0; c0 < 128; c0 += 16) {
+        for (int c0 = first_c; c0 < first_c + 64; c0 += 16) {
             float v[16];
             tc_ld16(t_dw + (uint32_t)c0, v);
 #pragma unroll
             for (int i = 0; i < 16; i += 4) put4(out + p_w + (part ? tt_quad(r, c0 + i, 128) : r * 128 + c0 + i), v + i);
         }
-        {
+        if (quarter % 2 == 0) {
             float v[16];
-            tc_ld16(t_row + (half == 0 ? TT_DW1 : TT_DW4), v);
-            if (half == 0) {
+            tc_ld16(t_row + (quarter == 0 ? TT_DW1 : TT_DW4), v);
+            if (quarter == 0) {
 #pragma unroll
                 for (int i = 0; i < 16; i += 4) put4(out + P_W1 + (part ? tt_quad(r, i, 128) : r * 16 + i), v + i);
             } else {
@@ -408,9 +423,12 @@ __global__ void __launch_bounds__(TT_THREADS, 1) fs_mlp_train_tc_kernel(
     }
     if (!ok && tid == 0 && part) part[(size_t)blockIdx.x * TT_PART + FS_MLP_NPARAM] = __int_as_float(0x7FC00000);
     if (!ok && tid == 0 && !part && loss_out) atomicAdd(loss_out, __int_as_float(0x7FC00000));  // gave up: NaN loss
-    // release the tensor memory once no MMA is in flight: after a give-up, wait (bounded)
-    // for the last commit's phase before freeing the columns
-    if (!ok) tc_wait(mbar, phase ^ 1u);
+    // release the tensor memory once no MMA is in flight: after a give-up, one more commit behind
+    // all of them, waited for (bounded) before freeing the columns
+    if (!ok) {
+        if (tid == 0) tc_commit(tc_smem(&S.mbar_last));
+        tc_wait(tc_smem(&S.mbar_last), 0u);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -449,8 +467,10 @@ __global__ void fs_mlp_adam_kernel(float *params, float *m, float *v, float *gra
 }
 
 // Adam step on the gradient that n_parts CTAs of the training pass left in their rows of part,
-// added in the CTAs' order.  The last thread adds the losses.
-__global__ void fs_mlp_adam_parts_kernel(const float *__restrict__ part, int n_parts, float *params, float *m, float *v,
+// added in the CTAs' order.  The last thread adds the losses.  Launched while the pass still runs
+// (params, m and v are not its to write); part is no read-only memory, so no load of it may move
+// above the wait.
+__global__ void fs_mlp_adam_parts_kernel(const float *part, int n_parts, float *params, float *m, float *v,
                                          fs_bf16 *wq, float lr, float b1c, float b2c, float *loss_out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -462,6 +482,7 @@ __global__ void fs_mlp_adam_parts_kernel(const float *__restrict__ part, int n_p
     else if (i >= P_W3 && i < P_B3) p = P_W3 + (i - P_W3) % 512 / 4 * 128 + (i - P_W3) / 512 * 4 + i % 4;
     const bool param = i < FS_MLP_NPARAM;
     const float w0 = param ? params[p] : 0.f, m0 = param ? m[p] : 0.f, v0 = param ? v[p] : 0.f;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the training pass has ended
     float g = 0.f;
 #pragma unroll 16
     for (int k = 0; k < n_parts; k++) g = __fadd_rn(g, part[(size_t)k * TT_PART + i]);
@@ -593,8 +614,18 @@ extern "C" int fs_mlp_train_batch(float *params, float *m, float *v, uint16_t *w
                         workspace, ctas, stream);
     if (rc) return rc;
     const float b1c = 1.f - powf(0.9f, (float)step), b2c = 1.f - powf(0.999f, (float)step);
-    fs_mlp_adam_parts_kernel<<<FS_MLP_NPARAM / 128 + 1, 128, 0, (cudaStream_t)stream>>>(
-        workspace, ctas, params, m, v, (fs_bf16 *)wq, lr, b1c, b2c, loss);
+    cudaLaunchAttribute early = {};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t at = {};
+    at.gridDim = dim3(FS_MLP_NPARAM / 128 + 1);
+    at.blockDim = dim3(128);
+    at.stream = (cudaStream_t)stream;
+    at.attrs = &early;
+    at.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&at, fs_mlp_adam_parts_kernel, (const float *)workspace, (int)ctas, params, m, v,
+                                       (fs_bf16 *)wq, lr, b1c, b2c, loss);
+    if (e != cudaSuccess) return fsi_thread_error(FS_ERR_LAUNCH, cudaGetErrorString(e));
     return launch_check("fs_mlp_adam_parts_kernel");
 }
 
