@@ -1381,8 +1381,13 @@ extern "C" int fs_run_host(fs_handle *h, const void *paths_in, void *paths_out, 
     const fs_config &c = h->cfg;
     CUDA_TRY(h, cudaSetDevice(h->device), FS_ERR_CUDA);
     if (n_chunks == 0) {
-        // automatic: as many chunks (up to 4) as still give every chunk half a wave of
-        // resident CTAs; small grids run as one chunk
+        // automatic: one chunk per half wave of resident CTAs and one to two more, up to 6; grids
+        // of less than a quarter wave run as one chunk.  A chunk more hides another part of the
+        // copies; a smaller one leaves SMs idle at its end, and its copies and events cost about 30 us.
+        // Trimers, us a call for 1 / 2 / 3 / 4 / 6 / 8 chunks (half waves): N = 128, 1000 walkers (0.2) 175 /
+        // 176 / 278 / 287 / 390 / 513; 2500 (0.5) 290 / 266 / 317 / 349 / 411 / 529; 5000 (1) 509 / 450 / 473 / 514 /
+        // 609 / 734; 16384 (3.4) 1416 / 1167 / 1119 / 1035 / 1023 / 1191; N = 256, 5000 walkers (2.1) 909 /
+        // 768 / 717 / 742 / 813 / 948; 16384 (6.7) 2742 / 2254 / 2058 / 1986 / 1891 / 1894.
         if (!h->resident_per_sm) {
             int per_sm = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)h->k_metro, h->block, h->smem) !=
@@ -1390,8 +1395,8 @@ extern "C" int fs_run_host(fs_handle *h, const void *paths_in, void *paths_out, 
                 cudaGetLastError();
             h->resident_per_sm = std::max(per_sm, 1);
         }
-        const long long half_wave = std::max(1ll, (long long)h->resident_per_sm * device_sms() / 2);
-        n_chunks = (int)std::max(1ll, std::min(4ll, (long long)h->grid / half_wave));
+        const long long wave = (long long)h->resident_per_sm * device_sms();
+        n_chunks = (int)std::min(6ll, (4ll * h->grid + 3 * wave) / (2 * wave));
     }
     h->idle = false;
     if (h->d_snap) n_chunks = 1;
