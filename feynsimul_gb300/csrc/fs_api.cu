@@ -833,10 +833,10 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         // builds) with at most 4 lags per thread run every lag in one pass over the slice
         // values, stored twice in a row so that slice s1 + tau needs no wrap.
         // Correlator helpers: a walker of at most 32 segment threads gets extra threads for
-        // the lag sums, up to 64 lag threads per walker (FS_MX in fs_pimc.cuh).  They need
-        // every CTA full (the walker count a multiple of the walkers per CTA, chosen below).
-        // Where the movers of a CTA fill whole warps (walker count and walkers per CTA
-        // multiples of 32 / threads per walker) the helpers are pipelined (FS_PIPE): the
+        // the lag sums, up to 64 lag threads per walker (FS_MX in fs_pimc.cuh).  Summing
+        // after the moves, they need every CTA full (the walker count a multiple of the walkers
+        // per CTA, chosen below).  Where the movers of a CTA fill whole warps (walkers per CTA a
+        // multiple of 32 / threads per walker) the helpers are pipelined (FS_PIPE): the
         // movers copy their slices to a double-buffered path snapshot, and the helpers alone
         // evaluate the correlator values on it and sum the lags, one measurement behind the
         // moves.
@@ -934,9 +934,8 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         h->wpb = c.walkers_per_block;
     } else if (h->mx > 1) {
         // CTAs of about 128 threads (moving and summing), every CTA full; pipelined: the
-        // movers in whole warps
-        // pipelined: the movers in whole warps, as few walkers per CTA as that allows (the
-        // CTAs spread evenly over the SMs)
+        // movers in whole warps, as few walkers per CTA as that allows (the CTAs spread evenly
+        // over the SMs)
         const int step = h->pipe ? 32 / h->tpw : 1;
         h->wpb = h->pipe ? step : std::max(1, 128 / (h->tpw * h->mx));
         while (h->wpb > step && (c.n_walkers % h->wpb || per_walker * h->wpb + hist_bytes > 100 * 1024))

@@ -228,8 +228,8 @@ __device__ __forceinline__ void fs_batch_tile(const FsBatchSys &sd, int tile, fl
                         // the degrees of freedom
                         auto node_x = [&](int d, float angle, float v) {
                             float rz = __fmul_rn(__fmul_rn(sig, sqrtf(__fmul_rn(-2.f, __logf(v)))), __sinf(angle));
-                            rz = v != 0.f ? rz : 0.f;
-                            FSB_AT(P, d, m) = __fadd_rn(__fmul_rn(0.5f, __fadd_rn(FSB_AT(P, d, l), FSB_AT(P, d, r))), rz);
+                            if (!FSB_RANLUX) rz = v != 0.f ? rz : 0.f;  // a RANLUX value is at least 2^-48
+                            FSB_AT(P, d, m) = __fmaf_rn(0.5f, __fadd_rn(FSB_AT(P, d, l), FSB_AT(P, d, r)), rz);
                         };
 #if FSB_RANLUX
                         // twelve values at a time, as the sweep's moves

@@ -7,8 +7,8 @@
 //   W1[128][16] b1[128] W2[128][128] b2[128] W3[128][128] b3[128] W4[16][128] b4[16]
 // The forward pass keeps the BF16 activations in shared memory; the loss gradient is formed
 // per row; the backward pass runs dA = dZ W and dW = dZ^T A and adds the weight / bias
-// gradients to an FP32 gradient array with atomics (the Adam kernel divides nothing: the
-// loss is already a batch mean).
+// gradients to an FP32 gradient array with atomics, or leaves each CTA's own for the optimiser to
+// add in order (the Adam kernel divides nothing: the loss is already a batch mean).
 //
 // Loss (per row, D degrees of freedom, z the midpoint's displacement from the endpoints'
 // mean in units of sigma_1): sum_d 0.5 (z_d - o_d)^2 exp(-s_d) + 0.5 s_d with
@@ -62,9 +62,9 @@ __device__ __forceinline__ fs_bf16 f2bf(float x)
 // columns): the layer accumulator F (a forward layer's output or a hidden gradient dA), and
 // the weight gradients summed over the CTA's tiles: dW2 and dW3 (128 columns each), dW1 (16)
 // and dW4 transposed (16; its M is the 128 inputs).  Shared memory holds BF16 tiles in the
-// canonical layout of fs_tc.cuh: the activations a1..a3 and the hidden gradient g (in turn g, a3
-// and g again, each 128 x 128, rows = the tile's rows), the input x and the output gradient dz4 (128 x 16), and the
-// weights W1..W4 ([out][in]).  The forward GEMMs read them K-major; dA = dZ W reads W
+// canonical layout of fs_tc.cuh: the activations a1..a3 and the hidden gradient (in g, then a3, then
+// g again), 128 x 128 each with the tile's rows, the input x and the output gradient dz4 (128 x
+// 16), and the weights W1..W4 ([out][in]).  The forward GEMMs read them K-major; dA = dZ W reads W
 // MN-major, and dW = dZ^T A reads dZ and A MN-major (K = the tile's rows), so no tile is
 // transposed.  The six 128-wide tiles come first and the allocation is padded, so every
 // byte a descriptor can reach lies inside it under either reading of its byte offsets.

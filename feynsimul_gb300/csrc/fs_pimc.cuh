@@ -35,7 +35,7 @@
 // operators and copy their slices into a double-buffered path snapshot (FS_SNSTRIDE words
 // each, the padded slice layout); the helper groups evaluate the correlator values on the
 // snapshot and sum the lags, for measurement m while the movers sweep towards measurement
-// m + 1.  One CTA barrier per measurement hands a snapshot over; the movers sync among
+// m + 1.  A helper lane sums FS_PLAGS consecutive lags.  One CTA barrier per measurement hands a snapshot over; the movers sync among
 // themselves on named barrier 1 and the helpers on named barrier 2.  Every sum is formed in
 // the same order as without the pipeline, so the results are the same bit for bit.
 #ifndef FS_MX
@@ -181,6 +181,7 @@
 #define FS_ADD __dadd_rn
 #define FS_SUB __dsub_rn
 #define FS_MUL __dmul_rn
+#define FS_FMA __fma_rn
 #define FS_DIV __ddiv_rn
 #define FS_SQRT_RN __dsqrt_rn
 #define FS_LOG log
@@ -192,6 +193,7 @@
 #define FS_ADD __fadd_rn
 #define FS_SUB __fsub_rn
 #define FS_MUL __fmul_rn
+#define FS_FMA __fmaf_rn
 #define FS_DIV __fdiv_rn
 #define FS_SQRT_RN __fsqrt_rn
 #if FS_FAST
@@ -206,6 +208,13 @@
 #define FS_SQRT sqrtf
 #define FS_TWO_PI 6.28318548f  // 2 * float(pi), as the reference's single-precision constant
 #endif
+
+// A proposed node, (l + r) / 2 + rz: halving is exact (a sum whose half is
+// subnormal aside), so the fused form has the same bits, an instruction a coordinate less (with
+// the next line, trimer, luxury 2: 5114 -> 5002 us a run, luxury 0 4153 -> 4023)
+#define FS_NODE(l, r, rz) FS_FMA((FT)0.5, FS_ADD(l, r), rz)
+// RANLUX values are at least 2^-48 (fs_rl_value), so only xorshift's v can be 0
+#define FS_V_POSITIVE (FS_RANLUX && !FS_DOUBLE)
 
 // 2 pi times a generator value in its own unit (fs_rng.cuh): the same product, one rounding
 #define FS_RAW_ANGLE (6.28318548f * FS_RL_UNIT)
@@ -364,8 +373,7 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
             // 64, where the twelve values spill (10 atoms, N = 1024 in device memory: 3830 against 3920)
             auto node_x = [&](int d, float angle, float v) {
                 float rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(angle));
-                rz = v != 0.0f ? rz : 0.0f;
-                FS_AT(P, d, m) = FS_ADD(FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r))), rz);
+                FS_AT(P, d, m) = FS_NODE(FS_AT(P, d, l), FS_AT(P, d, r), rz);
             };
 #pragma unroll 1
             for (int d0 = 0; d0 + 6 <= FS_DOF; d0 += 6) {
@@ -414,8 +422,8 @@ __device__ __forceinline__ int fs_bisect(FT *P, FT *Vc, fs_u32 start, FsUStream 
                 // is -inf, so that lane's product is infinite or NaN and is discarded, and no
                 // branch is taken per degree of freedom.
                 FT rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(angle));
-                rz = v != (FT)0 ? rz : (FT)0;
-                FS_AT(P, d, m) = FS_ADD(FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r))), rz);
+                if (!FS_V_POSITIVE) rz = v != (FT)0 ? rz : (FT)0;
+                FS_AT(P, d, m) = FS_NODE(FS_AT(P, d, l), FS_AT(P, d, r), rz);
             }
 #endif
         }
@@ -559,9 +567,9 @@ __device__ __forceinline__ int fs_bisect_lanes(FT *P, FT *Vc, fs_u32 start, FsUS
                 const FT angle = FS_MUL((FT)FS_TWO_PI, u);
 #endif
                 FT rz = FS_MUL(FS_MUL(sig, FS_SQRT(FS_MUL((FT)-2, FS_LOG(v)))), FS_SIN(angle));
-                rz = v != (FT)0 ? rz : (FT)0;
+                if (!FS_V_POSITIVE) rz = v != (FT)0 ? rz : (FT)0;
                 if (FS_DOF % FS_G == 0 || d < FS_DOF)
-                    FS_AT(P, d, m) = FS_ADD(FS_MUL((FT)0.5, FS_ADD(FS_AT(P, d, l), FS_AT(P, d, r))), rz);
+                    FS_AT(P, d, m) = FS_NODE(FS_AT(P, d, l), FS_AT(P, d, r), rz);
             }
         }
     }
