@@ -34,6 +34,7 @@ EXPORTS = (
     "fs_zero_accumulators", "fs_get_run_time", "fs_rng_ranlux_stream", "fs_rng_ranlux_stream64",
     "fs_rng_xorshift_stream", "fs_version", "fs_ranlux_init_noalloc", "fs_set_correlator",
     "fs_set_bins", "fs_set_histogram", "fs_mlp_sizes", "fs_mlp_train_step", "fs_mlp_adam", "fs_mlp_train_batch", "fs_mlp_workspace",
+    "fs_mlp_train_rows",
     "fs_mlp_pack", "fs_mlp_infer", "fs_set_learned_proposal", "fs_batch_create", "fs_batch_destroy",
     "fs_batch_run", "fs_batch_sync", "fs_batch_get_run_time", "fs_batch_set_paths", "fs_batch_get_paths",
     "fs_batch_set_seeds", "fs_batch_init_ranlux", "fs_batch_get_ranlux_tables", "fs_batch_get_op_sums",
@@ -141,6 +142,7 @@ _PROTOS = {
     "fs_set_histogram": ([_P, _P, _S], ctypes.c_int),
     "fs_mlp_sizes": ([_P, _P, _P, _P], ctypes.c_int),
     "fs_mlp_train_step": ([_P, _P, _P, _P, _P, _I, _I, ctypes.c_float, _P, _P], ctypes.c_int),
+    "fs_mlp_train_rows": ([_P, _P, _P, _P, _P, _P, _I, _I, ctypes.c_float, _P, _P], ctypes.c_int),
     "fs_mlp_adam": ([_P, _P, _P, _P, _P, _I, ctypes.c_float, _P], ctypes.c_int),
     "fs_mlp_workspace": ([_I, _P], ctypes.c_int),
     "fs_mlp_train_batch": ([_P, _P, _P, _P, _P, _P, _P, _I, _I, _P, _I, ctypes.c_float, _P, ctypes.c_int64, _P],

@@ -197,9 +197,12 @@ class LearnedProposal:
         return float(np.mean(np.sum(0.5 * z * z - nll, axis=1)))
 
     # ---- training on the GPU with the project's kernels ----
-    def train(self, feats, targets, steps=2000, batch=4096, lr=1e-3, seed=0, log_every=0):
+    def train(self, feats, targets, steps=2000, batch=4096, lr=1e-3, seed=0, log_every=0, reproducible=False):
         """Adam on the Gaussian negative log-likelihood; returns the loss history (per step,
-        mean over the batch)."""
+        mean over the batch).  The gradients of a batch's 128-row tiles are added as they arrive
+        (fs_mlp_train_rows), so two calls may differ in the last bits of a step and, as Adam and the
+        BF16 weights carry that on, by 1e-4 to 1e-2 of the parameters after 20 to 100 steps.
+        reproducible=True adds them in order (fs_mlp_train_batch): equal calls give equal bits."""
         import torch
         L = _lib.lib()
         dev = "cuda"
@@ -212,9 +215,6 @@ class LearnedProposal:
         tp = torch.from_numpy(self.params.copy()).to(dev)
         tm = torch.zeros_like(tp)
         tv = torch.zeros_like(tp)
-        need = ctypes.c_int64()
-        _lib.check(L.fs_mlp_workspace(batch, ctypes.byref(need)))
-        work = torch.empty(need.value, dtype=torch.float32, device=dev)
         tq = torch.zeros(n_bf16, dtype=torch.int16, device=dev)
         frag_dummy = torch.zeros(sizes[2].value * 2, dtype=torch.int32, device=dev)
         bias_dummy = torch.zeros(sizes[3].value, dtype=torch.float32, device=dev)
@@ -225,13 +225,25 @@ class LearnedProposal:
         gen = torch.Generator(device=dev)
         gen.manual_seed(seed)
         sums = torch.zeros(steps, dtype=torch.float32, device=dev)  # each step's loss over its batch
-        before_rows = tp.data_ptr(), tm.data_ptr(), tv.data_ptr(), tq.data_ptr(), tx.data_ptr(), tz.data_ptr()
-        sum_ptr, work_ptr = sums.data_ptr(), work.data_ptr()
+        sum_ptr = sums.data_ptr()
+        if reproducible:
+            need = ctypes.c_int64()
+            _lib.check(L.fs_mlp_workspace(batch, ctypes.byref(need)))
+            work = torch.empty(need.value, dtype=torch.float32, device=dev)
+        else:
+            tg = torch.zeros_like(tp)
         for it in range(steps):
             # the training kernel gathers the batch's rows itself
             idx = torch.randint(0, n, (batch,), device=dev, generator=gen)
-            _lib.check(L.fs_mlp_train_batch(*before_rows, idx.data_ptr(), batch, self.dof, sum_ptr + 4 * it, it + 1, lr,
-                                            work_ptr, need.value, stream))
+            if reproducible:
+                _lib.check(L.fs_mlp_train_batch(tp.data_ptr(), tm.data_ptr(), tv.data_ptr(), tq.data_ptr(), tx.data_ptr(),
+                                                tz.data_ptr(), idx.data_ptr(), batch, self.dof, sum_ptr + 4 * it, it + 1,
+                                                lr, work.data_ptr(), need.value, stream))
+            else:
+                _lib.check(L.fs_mlp_train_rows(tp.data_ptr(), tq.data_ptr(), tg.data_ptr(), tx.data_ptr(), tz.data_ptr(),
+                                               idx.data_ptr(), batch, self.dof, 1.0 / batch, sum_ptr + 4 * it, stream))
+                _lib.check(L.fs_mlp_adam(tp.data_ptr(), tm.data_ptr(), tv.data_ptr(), tg.data_ptr(), tq.data_ptr(),
+                                         it + 1, lr, stream))
             if log_every and (it + 1) % log_every == 0:
                 print(f"step {it + 1}: loss {float(sums[it] / batch):.4f}")
         losses = sums / batch

@@ -312,6 +312,11 @@ int fs_mlp_sizes(int64_t *n_param, int64_t *n_bf16, int64_t *n_frag_u2, int64_t 
 int fs_mlp_train_step(const float *params, const uint16_t *wq, float *grad, const float *x,
                       const float *z, int32_t n_rows, int32_t dof, float inv_batch, float *loss,
                       void *stream);
+/* fs_mlp_train_step on the rows of a training set that `rows` (device, n_rows numbers, each within
+ * the set) picks, gathered in place. */
+int fs_mlp_train_rows(const float *params, const uint16_t *wq, float *grad, const float *x,
+                      const float *z, const int64_t *rows, int32_t n_rows, int32_t dof,
+                      float inv_batch, float *loss, void *stream);
 /* Adam (beta 0.9 / 0.999) on params; refreshes the BF16 copy wq; clears grad. */
 int fs_mlp_adam(float *params, float *m, float *v, float *grad, uint16_t *wq, int32_t step,
                 float lr, void *stream);
