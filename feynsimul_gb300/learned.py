@@ -203,10 +203,14 @@ class LearnedProposal:
         (fs_mlp_train_rows), so two calls may differ in the last bits of a step and, as Adam and the
         BF16 weights carry that on, by 1e-4 to 1e-2 of the parameters after 20 to 100 steps.
         reproducible=True adds them in order (fs_mlp_train_batch): equal calls give equal bits."""
+        fs, ts = tuple(np.shape(feats)), tuple(np.shape(targets))
+        if len(fs) != 2 or fs[1] != IN or len(ts) != 2 or ts[1] != 8 or ts[0] < fs[0]:
+            # the kernel reads 16 and 8 values of any row below n
+            raise ValueError(f"train needs feats (n, {IN}) and targets (n, 8), got {fs} and {ts}")
+        n = fs[0]
         import torch
         L = _lib.lib()
         dev = "cuda"
-        n = feats.shape[0]
         batch = min(batch, n)
         sizes = [ctypes.c_int64() for _ in range(4)]
         _lib.check(L.fs_mlp_sizes(*[ctypes.byref(v) for v in sizes]))
