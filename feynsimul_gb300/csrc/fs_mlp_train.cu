@@ -472,14 +472,15 @@ __global__ void fs_mlp_adam_kernel(float *params, float *m, float *v, float *gra
 }
 
 // Adam step on the gradient that n_parts CTAs of the training pass left in their rows of part,
-// added in the CTAs' order.  The last thread adds the losses.  Launched while the pass still runs
+// added in the CTAs' order.  The last thread adds the losses.  A CTA that gave up has written no
+// gradient, only a NaN for its loss: with any such loss the step leaves the parameters, moments and
+// weights as they are.  Launched while the pass still runs
 // (params, m and v are not its to write); part is no read-only memory, so no load of it may move
 // above the wait.
 __global__ void fs_mlp_adam_parts_kernel(const float *part, int n_parts, float *params, float *m, float *v,
                                          fs_bf16 *wq, float lr, float b1c, float b2c, float *loss_out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > FS_MLP_NPARAM) return;
     // the parameter at place i of the row (tt_quad)
     int p = i;
     if (i < P_B1) p = P_W1 + (i - P_W1) % 512 / 4 * 16 + (i - P_W1) / 512 * 4 + i % 4;
@@ -488,6 +489,13 @@ __global__ void fs_mlp_adam_parts_kernel(const float *part, int n_parts, float *
     const bool param = i < FS_MLP_NPARAM;
     const float w0 = param ? params[p] : 0.f, m0 = param ? m[p] : 0.f, v0 = param ? v[p] : 0.f;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the training pass has ended
+    bool nan = false;
+    for (int k = threadIdx.x; k < n_parts; k += blockDim.x) {
+        const float loss = part[(size_t)k * TT_PART + FS_MLP_NPARAM];
+        nan |= loss != loss;
+    }
+    nan = __syncthreads_or(nan);
+    if (i > FS_MLP_NPARAM || (nan && param)) return;
     float g = 0.f;
 #pragma unroll 16
     for (int k = 0; k < n_parts; k++) g = __fadd_rn(g, part[(size_t)k * TT_PART + i]);

@@ -252,8 +252,11 @@ class LearnedProposal:
                 print(f"step {it + 1}: loss {float(sums[it] / batch):.4f}")
         losses = sums / batch
         torch.cuda.synchronize()
-        self.params = tp.cpu().numpy().astype(np.float32)
-        hist = losses.cpu().numpy()
+        params, hist = tp.cpu().numpy().astype(np.float32), losses.cpu().numpy()
+        if np.isnan(hist).any() and np.isfinite(params).all():
+            # NaN data make the parameters NaN, except in order, where such a batch is left out
+            raise _lib.FsError(_lib.FS_ERR_LAUNCH, "a training pass gave up, or (reproducible=True) a batch's loss is NaN")
+        self.params = params
         self.history.extend(hist.tolist())
         return hist
 

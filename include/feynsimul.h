@@ -324,7 +324,9 @@ int fs_mlp_adam(float *params, float *m, float *v, float *grad, uint16_t *wq, in
  * within the set) picks: the pass of fs_mlp_train_step over them with inv_batch = 1 / n_rows,
  * gathered in place, and the Adam step of fs_mlp_adam; *loss becomes the batch's loss sum.  The
  * CTAs' gradients pass through `workspace` (device, 16-byte aligned, fs_mlp_workspace floats) and
- * are added in order, so equal runs give equal bits. */
+ * are added in order, so equal runs give equal bits.  A batch whose loss is NaN (NaN among its
+ * rows' z, or a pass that gave up waiting for its tensor cores) leaves params, m, v and wq as they
+ * were. */
 int fs_mlp_workspace(int32_t n_rows, int64_t *n_floats);
 int fs_mlp_train_batch(float *params, float *m, float *v, uint16_t *wq, const float *x, const float *z,
                        const int64_t *rows, int32_t n_rows, int32_t dof, float *loss, int32_t step,

@@ -54,6 +54,10 @@ class _State:
         self.check(self.L.fs_mlp_pack(self.p.data_ptr(), self.q.data_ptr(), f.data_ptr(), b.data_ptr(), self.stream))
         self.loss = torch.zeros(1, dtype=torch.float32, device="cuda")
 
+    def copy_from(self, o):
+        for a in ("p", "m", "v", "q"):
+            getattr(self, a).copy_(getattr(o, a))
+
     def step(self, xb, zb, dof, it, lr=1e-3):
         self.loss.zero_()
         n = xb.shape[0]
@@ -138,3 +142,87 @@ def test_both_orders_are_as_exact(batch, dof):
     arrive = [_far(run()[1], exact) for _ in range(5)]
     ordered = _far(p1, exact)
     assert ordered <= 1.5 * max(arrive) and max(arrive) <= 1.5 * ordered
+
+
+def test_ordered_steps_reuse_their_workspace():
+    # more tiles than SMs, then fewer and fewer, on one workspace of NaN: every step uses only the
+    # rows its own CTAs wrote, and the optimiser, launched early, the moments of the step before
+    import torch
+    dof = 6
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    x, z = _data(40000, dof, 3)
+    tx, tz = torch.from_numpy(x).cuda(), torch.from_numpy(z).cuda()
+    rng = np.random.RandomState(4)
+    counts = [128 * sms + 300, 4096, 129, 1, 700, 128 * sms]
+    rows = [torch.from_numpy(rng.randint(0, x.shape[0], n)).cuda() for n in counts]
+    p0 = _network(dof, 3)
+    one = _State(p0)
+    need = ctypes.c_int64()
+    one.check(one.L.fs_mlp_workspace(max(counts), ctypes.byref(need)))
+    stride = need.value // sms
+
+    def run(look):
+        s, other = _State(p0), _State(p0)
+        work = torch.full((need.value,), math.nan, dtype=torch.float32, device="cuda")
+        out = []
+        for it, idx in enumerate(rows, 1):
+            if look:
+                other.copy_from(s)
+            s.check(s.L.fs_mlp_train_batch(s.p.data_ptr(), s.m.data_ptr(), s.v.data_ptr(), s.q.data_ptr(), tx.data_ptr(),
+                                           tz.data_ptr(), idx.data_ptr(), idx.numel(), dof, s.loss.data_ptr(), it, 1e-3,
+                                           work.data_ptr(), need.value, s.stream))
+            out.append((s.p.clone(), s.m.clone(), s.loss.clone()))
+            if look:  # the same step by atomics: FP32 sums of the same terms in another order
+                other.step(tx[idx], tz[idx], dof, it)
+                torch.cuda.synchronize()
+                n = min(-(-idx.numel() // 128), sms)
+                parts = work.cpu().numpy().astype(np.float64).reshape(sms, stride)[:n, :p0.size]
+                size = np.linalg.norm(np.abs(parts).sum(axis=0))
+                m, w = s.m.cpu().numpy().astype(np.float64), other.m.cpu().numpy().astype(np.float64)
+                assert np.linalg.norm(m - w) <= 2.0 ** -24 * (0.1 * (2 * n + 8) * size + 4 * np.linalg.norm(w))
+        torch.cuda.synchronize()
+        return out
+
+    for a, b in zip(run(True), run(False)):
+        for u, w in zip(a, b):
+            assert torch.equal(u, w)
+
+
+@pytest.mark.parametrize("rows", [1, 300, 20000])
+def test_ordered_step_without_a_loss_changes_nothing(rows):
+    # as after a pass that gave up: a NaN loss in one CTA's row of the workspace, the last one's
+    import torch
+    from feynsimul_gb300 import _lib
+    from feynsimul_gb300.learned import LearnedProposal
+    dof = 6
+    x, z = _data(rows, dof, 1)
+    p0 = _network(dof, 1)
+    s = _State(p0)
+    tx, tz = torch.from_numpy(x).cuda(), torch.from_numpy(z).cuda()
+    need = ctypes.c_int64()
+    s.check(s.L.fs_mlp_workspace(rows, ctypes.byref(need)))
+    work = torch.full((need.value,), math.nan, dtype=torch.float32, device="cuda")
+    idx = torch.arange(rows, device="cuda")
+
+    def step(it):
+        s.check(s.L.fs_mlp_train_batch(s.p.data_ptr(), s.m.data_ptr(), s.v.data_ptr(), s.q.data_ptr(), tx.data_ptr(),
+                                       tz.data_ptr(), idx.data_ptr(), rows, dof, s.loss.data_ptr(), it, 1e-3,
+                                       work.data_ptr(), need.value, s.stream))
+        torch.cuda.synchronize()
+
+    step(1)
+    before = [t.clone() for t in (s.p, s.m, s.v, s.q)]
+    assert math.isfinite(float(s.loss[0])) and not np.array_equal(before[0].cpu().numpy(), p0)
+    tz[rows - 1, 0] = math.nan
+    step(2)
+    assert math.isnan(float(s.loss[0]))
+    for a, b in zip(before, (s.p, s.m, s.v, s.q)):
+        assert torch.equal(a, b)
+
+    z[rows - 1, 0] = math.nan
+    m = LearnedProposal(dof, 0.25, 5.0, params=p0)
+    with pytest.raises(_lib.FsError, match="NaN"):
+        m.train(x, z, steps=5, batch=rows, seed=2, reproducible=True)  # 5 draws of `rows` of `rows` rows
+    assert np.array_equal(m.params, p0) and m.history == []
+    hist = m.train(x, z, steps=5, batch=rows, seed=2)  # as ever: NaN data give NaN parameters
+    assert np.isnan(hist).any() and np.isnan(m.params).any()
