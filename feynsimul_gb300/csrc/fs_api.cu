@@ -609,6 +609,30 @@ static size_t sweep_smem(const fs_handle &h, long long vstride, size_t hist_byte
     return (size_t)(path + round16(h.wpb * vstride) + h.wpb * h.cwstride) * h.ft + hist_bytes;
 }
 
+// What is left of a CTA's 227 KB beside the kernel's static shared memory: with RANLUX each walker's
+// offset stream (FsIStream: 26 words, 16 doublewords in FP64) and its offset, or a byte for every
+// step of the launch (FS_OFF_PRE).
+static size_t smem_room(const fs_handle &h, int wpb)
+{
+    const fs_config &c = h.cfg;
+    if (!c.enable_ranlux) return 227 * 1024;
+    const long long steps = (long long)c.operator_runs * c.metro_steps_per_operator_run;
+    const bool ahead = c.enable_parallelize_path && h.seg <= 256 && steps <= 256;
+    const size_t bytes = (size_t)wpb * ((c.enable_double ? 128 : 104) + (ahead ? (size_t)steps : 4));
+    return 227 * 1024 - std::min<size_t>(227 * 1024, (bytes + 15) / 16 * 16);
+}
+
+// The learned proposal's network is evaluated warp-wide, so every lane of every warp holds a walker:
+// wpb as a multiple of the 32 / T walkers of a warp that divides the walker count (itself such a
+// multiple, which prepare() checks).
+static int whole_warps(const fs_handle &h, int wpb)
+{
+    const int wpw = 32 / h.tpw;
+    wpb = std::max(wpw, wpb / wpw * wpw);
+    while (wpb > wpw && h.cfg.n_walkers % wpb) wpb -= wpw;
+    return wpb;
+}
+
 // Walkers per CTA of a sweep without correlator helpers: CTAs of 128 threads, at most 100 KB of
 // shared memory, and where the walkers are so few that some SMs would get no CTA, fewer per CTA
 // down to a warp of threads (444 bound trimers, 8 threads each: 747 us a run in 28 CTAs of 4
@@ -680,10 +704,11 @@ static bool path_in_shared(const fs_handle &h, size_t path_bytes, size_t hist_by
 {
     const fs_config &c = h.cfg;
     if (!h.cors.empty()) return false;
-    const int wpb = std::min(c.walkers_per_block > 0 ? c.walkers_per_block : default_wpb(h, path_bytes, hist_bytes),
-                             c.n_walkers);
+    int wpb = std::min(c.walkers_per_block > 0 ? c.walkers_per_block : default_wpb(h, path_bytes, hist_bytes),
+                       c.n_walkers);
+    if (c.learned) wpb = whole_warps(h, wpb);
     const size_t smem = path_bytes * wpb + 2 * 16 * h.ft + hist_bytes;
-    if (smem > 227 * 1024) return false;
+    if (smem > smem_room(h, wpb)) return false;
     const long long ctas = std::min((227ll * 1024) / (long long)(smem + 1024), 2048ll / (wpb * h.tpw * h.lanes));
     if (ctas < std::max(1, c.min_blocks_per_sm)) return false;
     return ctas * device_sms() * wpb >= c.n_walkers || ctas * wpb * h.tpw * h.lanes >= 384;
@@ -957,14 +982,12 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         return fail(nullptr, FS_ERR_CONFIG, "internal: threads per walker must divide 32");
     }
     if (c.learned) {
-        // the network is evaluated warp-wide: every lane of every warp must hold a walker
         const int wpw = 32 / h->tpw;
-        h->wpb = std::max(wpw, (h->wpb / wpw) * wpw);
         if (c.n_walkers % wpw) {
             delete h;
             return fail(nullptr, FS_ERR_CONFIG, "the learned proposal needs the walker count to be a multiple of %d", wpw);
         }
-        while (c.n_walkers % h->wpb) h->wpb -= wpw;
+        h->wpb = whole_warps(*h, h->wpb);
     }
     h->block = h->wpb * h->tpw * h->lanes * h->mx;
     if (h->block > 1024) {
@@ -973,6 +996,7 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
     }
     h->grid = (c.n_walkers + h->wpb - 1) / h->wpb;
     h->smem = sweep_smem(*h, h->vstride, hist_bytes);
+    const size_t room = smem_room(*h, h->wpb);
     if (h->vstride && c.potential_cache == 0) {
         // automatic: the cache halves the potential evaluations but takes shared memory;
         // keep it where it costs no resident CTA per SM, or where the potential is large
@@ -981,7 +1005,7 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         const size_t without = sweep_smem(*h, 0, hist_bytes);
         if (ctas(h->smem) < std::min(ctas(without), 2048ll / h->block) && c.dof <= 8) h->vstride = 0;
     }
-    if (h->smem > 227 * 1024 && h->vstride && c.potential_cache != 1) h->vstride = 0;  // no room
+    if (h->smem > room && h->vstride && c.potential_cache != 1) h->vstride = 0;
     if (!h->vstride) {
         h->smem = sweep_smem(*h, 0, hist_bytes);
         // automatic: where shared memory has no room for the cache, keep it in device memory
@@ -991,7 +1015,7 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
             (long long)c.operator_runs * c.metro_steps_per_operator_run >= 2)
             h->vglobal = 1;
     }
-    if (h->smem > 227 * 1024) {
+    if (h->smem > room) {
         // the bank spread is not worth a CTA that fits without it
         if (!c.global_path) h->wstride = round16((long long)c.dof * dstride);
         if (h->vstride) h->vstride = round16(dstride);
@@ -1018,11 +1042,11 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
         h->cfg.min_blocks_per_sm =
             (int)std::max(1ll, std::min(std::min(std::min(by_smem, by_threads), by_regs), by_grid));
     }
-    if (h->smem > 227 * 1024) {
+    if (h->smem > room) {
+        const size_t bytes = h->smem;
         delete h;
         return fail(nullptr, FS_ERR_CONFIG,
-                    "a walker's path does not fit in shared memory (%zu bytes per CTA); lower walkers_per_block",
-                    h->smem);
+                    "a walker's path does not fit in shared memory (%zu bytes per CTA); lower walkers_per_block", bytes);
     }
 
     // ---- source + compile ----
