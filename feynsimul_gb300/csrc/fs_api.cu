@@ -686,6 +686,7 @@ static int lanes_for(const fs_handle &h)
                 {2, dbl ? 1.0 : ranlux ? 1.6 : 2.0}};
     for (const auto &r : rule) {
         if (r.lanes > h.seg || r.lanes * h.tpw > 1024 || warps * r.lanes > r.most * schedulers) continue;
+        if (c.min_blocks_per_sm * r.lanes * h.tpw > 2048) continue;  // the caller's CTAs per SM
         if (c.dof <= 8 && (r.lanes > h.seg / 2 || (h.seg < 8 && r.lanes * h.tpw > 32))) continue;
         return r.lanes;
     }

@@ -19,6 +19,15 @@ def test_learned_walkers_in_device_memory_compile():
     assert rc == 0, log
 
 
+@pytest.mark.parametrize("N,S,per_sm", [(1024, 3, 8), (2048, 4, 4), (1024, 3, 16)])
+def test_lanes_leave_the_callers_register_budget(N, S, per_sm):
+    # three walkers would take 4 or 8 lanes a segment thread: CTAs that no SM holds per_sm of, for
+    # which ptxas drops the budget
+    rc, log = _compile(_cfg(dof=6, n_slices=N, bisection_level=S, n_walkers=3, min_blocks_per_sm=per_sm), _quadratic(6),
+                       "", ("x1 * x1",))
+    assert rc == 0 and "will be ignored" not in log, log
+
+
 def test_refused_size_is_named():
     rc, log = _compile(_cfg(dof=9, n_slices=512, bisection_level=9, walkers_per_block=16), _quadratic(9))
     assert rc == -1 and "does not fit in shared memory (" in log
