@@ -174,7 +174,7 @@
 #endif
 // a move keeps its old cached values (FS_SEG - 1 of them) for a rejection
 #ifndef FS_VKEEP
-#define FS_VKEEP (FS_SEG <= 33)
+#define FS_VKEEP (FS_SEG > 1 && FS_SEG <= 33)
 #endif
 
 #if FS_DOUBLE

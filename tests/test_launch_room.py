@@ -28,6 +28,16 @@ def test_lanes_leave_the_callers_register_budget(N, S, per_sm):
     assert rc == 0 and "will be ignored" not in log, log
 
 
+@pytest.mark.parametrize("dof,kw", [
+    (2, dict(n_slices=4, potential_cache=1)), (9, dict(n_slices=256)), (3, dict(n_slices=8, potential_cache=3, enable_ranlux=1)),
+    (6, dict(n_slices=64, metro_steps_per_operator_run=0)), (1, dict(n_slices=8, potential_cache=1, enable_parallelize_path=0)),
+])
+def test_level_zero_compiles(dof, kw):
+    # a move without nodes: no cached values to keep for a rejection
+    rc, log = _compile(_cfg(dof=dof, bisection_level=0, n_walkers=64, **kw), _quadratic(dof), "", ("x1 * x1",))
+    assert rc == 0, log
+
+
 def test_refused_size_is_named():
     rc, log = _compile(_cfg(dof=9, n_slices=512, bisection_level=9, walkers_per_block=16), _quadratic(9))
     assert rc == -1 and "does not fit in shared memory (" in log
