@@ -617,7 +617,7 @@ static size_t smem_room(const fs_handle &h, int wpb)
     const fs_config &c = h.cfg;
     if (!c.enable_ranlux) return 227 * 1024;
     const long long steps = (long long)c.operator_runs * c.metro_steps_per_operator_run;
-    const bool ahead = c.enable_parallelize_path && h.seg <= 256 && steps <= 256;
+    const bool ahead = c.enable_parallelize_path && h.seg <= 256 && steps > 0 && steps <= 256;
     const size_t bytes = (size_t)wpb * ((c.enable_double ? 128 : 104) + (ahead ? (size_t)steps : 4));
     return 227 * 1024 - std::min<size_t>(227 * 1024, (bytes + 15) / 16 * 16);
 }

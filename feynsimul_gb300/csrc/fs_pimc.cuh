@@ -881,7 +881,7 @@ __device__ __forceinline__ void fs_flag_nonfinite(int *status, int walker)
 // the steps read them: the same draws in the same order, and the generator's code for that
 // stream stays out of the move loop.
 #define FS_NSTEPS_LAUNCH (FS_OPRUNS * FS_MSTEPS)
-#if FS_RANLUX && FS_PARALLEL && FS_BISECT && FS_SEG <= 256 && FS_NSTEPS_LAUNCH <= 256
+#if FS_RANLUX && FS_PARALLEL && FS_BISECT && FS_SEG <= 256 && FS_NSTEPS_LAUNCH > 0 && FS_NSTEPS_LAUNCH <= 256
 #define FS_OFF_PRE 1
 #else
 #define FS_OFF_PRE 0

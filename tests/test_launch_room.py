@@ -38,6 +38,12 @@ def test_level_zero_compiles(dof, kw):
     assert rc == 0, log
 
 
+def test_measurements_without_moves_compile():
+    # metroStepsPerOperatorRun = 0: RANLUX has no offsets to draw ahead
+    rc, log = _compile(_cfg(enable_ranlux=1, metro_steps_per_operator_run=0), "0.5 * x1 * x1", "", ("x1 * x1",))
+    assert rc == 0, log
+
+
 def test_refused_size_is_named():
     rc, log = _compile(_cfg(dof=9, n_slices=512, bisection_level=9, walkers_per_block=16), _quadratic(9))
     assert rc == -1 and "does not fit in shared memory (" in log
