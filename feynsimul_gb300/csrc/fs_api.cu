@@ -1773,6 +1773,7 @@ extern "C" int fs_get_accepts(fs_handle *h, uint32_t *out, size_t n)
     if (!h->h_accepts) return copy_out(h, out, h->d_accepts, n * 4, (size_t)h->n_threads * 4);
     if (n != (size_t)h->n_threads)
         return fail(h, FS_ERR_IO, "buffer has %zu bytes, expected %zu", n * 4, (size_t)h->n_threads * 4);
+    if (!out) return fail(h, FS_ERR_CONFIG, "null buffer");
     CUDA_TRY(h, drain(h), FS_ERR_LAUNCH);
     memcpy(out, h->h_accepts, n * 4);
     return FS_OK;

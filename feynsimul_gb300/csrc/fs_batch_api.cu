@@ -540,6 +540,7 @@ static int sys_copy(fs_batch *b, int32_t i, void *dev, void *host, size_t bytes,
 static int host_copy(fs_batch *b, const void *src, void *out, size_t bytes, size_t expect)
 {
     if (bytes != expect) return bfail(FS_ERR_IO, "buffer has %zu bytes, expected %zu", bytes, expect);
+    if (!out) return bfail(FS_ERR_CONFIG, "null buffer");
     int rc = drain(b);
     if (!rc) memcpy(out, src, bytes);
     return rc;
