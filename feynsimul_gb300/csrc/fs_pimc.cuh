@@ -76,8 +76,9 @@
 #define FS_LAG(j) (lt + (j) * FS_CTPW)
 #endif
 // Helpers and movers share CTA barriers, so every thread of a CTA has to run.  Where the walkers do
-// not fill the last CTA (FS_RAGGED, pipelined helpers only), its spare threads run on a path of
-// zeros and the last walker's generator rows, and write nothing to device memory.
+// not fill the last CTA (FS_RAGGED, pipelined helpers only), its spare threads run along as the last
+// walker, on copies of its path and generator rows, and write nothing to device memory: a plugin
+// sees no coordinates that a walker has not got.
 #define FS_RAGGED (FS_PIPE && FS_NWALKERS % FS_WPB != 0)
 #if FS_MX > 1 && (!FS_PARALLEL || FS_TPW > 32 || FS_GLOBAL || FS_NCOR == 0 || (FS_NWALKERS % FS_WPB != 0 && !FS_RAGGED))
 #error "correlator helpers need parallel-path walkers of at most 32 threads in shared memory, correlators, and full CTAs"
@@ -933,7 +934,7 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
     {
 #if !FS_GLOBAL
         const size_t base = (size_t)w0 * FS_DOF * FS_N;
-        const int count = n_here * FS_DOF * FS_N;
+        const int count = (FS_RAGGED ? FS_WPB : n_here) * FS_DOF * FS_N;
 #if FS_VEC > 1
         // 16-byte loads of FS_VEC consecutive slices; they lie in one 2^S block of the padded
         // layout, so their shared-memory words are consecutive too
@@ -943,19 +944,17 @@ extern "C" __global__ void FS_LAUNCH_BOUNDS fs_metropolis(FsArgs a)
             const int wi = i / (FS_DOF * FS_N), r = i - wi * (FS_DOF * FS_N);
             const int d = r / FS_N, sl = r - d * FS_N;
             FT *dst = &FS_AT(s_path + wi * FS_WSTRIDE, d, sl);
-            const FsVec v = src[i4];
+            const FsVec v = src[FS_RAGGED ? (min(wi, n_here - 1) * (FS_DOF * FS_N) + r) / FS_VEC : i4];
             fs_vec_scatter(dst, v);
         }
 #else
         for (int i = tid_b; i < count; i += FS_BLOCK) {
             const int wi = i / (FS_DOF * FS_N), r = i - wi * (FS_DOF * FS_N);
             const int d = r / FS_N, sl = r - d * FS_N;
-            FS_AT(s_path + wi * FS_WSTRIDE, d, sl) = a.paths[base + i];
+            FS_AT(s_path + wi * FS_WSTRIDE, d, sl) =
+                a.paths[base + (FS_RAGGED ? min(wi, n_here - 1) * (FS_DOF * FS_N) + r : i)];
         }
 #endif
-#endif
-#if FS_RAGGED
-        for (int i = n_here * FS_WSTRIDE + tid_b; i < FS_WPB * FS_WSTRIDE; i += FS_BLOCK) s_path[i] = (FT)0;
 #endif
 #if FS_NHIST > 0
         for (int i = tid_b; i < FS_HBINS; i += FS_BLOCK) s_hist[i] = 0u;
