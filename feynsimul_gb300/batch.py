@@ -45,7 +45,9 @@ def choose_S(N, tpw_target, block, dof=None, smem_budget=200 * 1024):
     walker gets up to the whole CTA (segments of at least 4 slices), so the tile does not
     leave warps idle at its barriers.  With segments of at least 8 slices, five of the
     standard workload's system types left 64-256 of a 512-thread CTA idle: 5.76e9 against
-    6.44e9 node updates/s with 4."""
+    6.44e9 node updates/s with 4.  The sizes here, a word of padding every 8 slices and 200 KB, are
+    an earlier tile's (now no padding and 226 KB): they stay, since a system's level decides its
+    streams and moves, and so its numbers."""
     S = int(np.log2(N)) - int(np.log2(tpw_target))
     S = max(1, min(S, 10, int(np.log2(N))))
     if dof is not None:
@@ -175,7 +177,7 @@ class BatchSampler:
 
 
 # bumped when the batch kernel or its launch-shape rules change, so cached tunings expire
-_TUNING_VERSION = 4
+_TUNING_VERSION = 5
 
 
 def _signature(workload, op_runs, msteps):
