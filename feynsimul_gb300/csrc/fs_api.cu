@@ -1185,7 +1185,10 @@ extern "C" int fs_destroy(fs_handle *h)
 {
     if (!h) return FS_OK;
     cudaSetDevice(h->device);
-    if (h->stream) cudaStreamSynchronize(h->stream);
+    // all of them: a host-buffer run that failed half-way has not joined its streams, and the page-locked
+    // block goes to the next handle without the device-wide wait of cudaFree
+    for (cudaStream_t st : {h->stream, h->s_in, h->s_comp2, h->s_out})
+        if (st) cudaStreamSynchronize(st);
     free_buffers(h);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
