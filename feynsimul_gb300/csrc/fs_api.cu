@@ -1709,9 +1709,10 @@ extern "C" int fs_get_walker_operators(fs_handle *h, double *out, size_t n)
 __global__ void fs_walker_ops_study_kernel(const double *ops, int n_walkers, int tpw, int wpg, int nwg, int nops,
                                            int parallel, double *out)
 {
-    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) / 32), lane = threadIdx.x % 32;
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x % 32;
     if (w >= n_walkers) return;
-    const long long first = parallel ? (long long)(w / wpg) * tpw + (long long)(w % wpg) * nwg * tpw : w;
+    const long long first = parallel ? w / wpg * tpw + w % wpg * nwg * tpw : w;
     for (int op = 0; op < nops; op++) {
         double s[3] = {0.0, 0.0, 0.0};
         for (int t = lane; t < tpw; t += 32)
