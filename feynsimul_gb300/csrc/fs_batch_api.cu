@@ -198,11 +198,28 @@ extern "C" int fs_batch_create(int32_t n_types, const int32_t *type_dof, const c
         *global = wpb * tpw * 2 < block_threads && dof > 8;
         return *global ? most : wpb;
     };
-    // CTAs per SM: 512 threads at the kernel's 128 registers, so a smaller CTA leaves shared memory
+    // Registers a thread: 128, which keep old segments of up to 112 values, or 64 and twice the CTAs on an
+    // SM, for xorshift batches of at most five atoms whose segments are small (30 values: four at level 2) and whose
+    // threads are many: more than a wave of 512-thread CTAs, four of smaller ones (CTAs below 256 threads
+    // gain none).  Us a launch at 128 / 64, 256 and 512 threads: 6000 walkers, 3 atoms, N = 256, level 2 172 /
+    // 148 and 184 / 161; 4 atoms, N = 128, level 1 137 / 108 and 147 / 121; 5 atoms 173 / 143 and 184 / 162; 1500
+    // walkers, 3 atoms, level 2 56 / 68 and 76 / 68; level 3, 4 atoms, 6000 241 / 310 and 295 / 312.
+    long long threads = 0;
+    bool small = b->lux < 0 && block_threads >= 256 && block_threads <= 512, deep = false;
+    for (const fs_batch_system &s : b->sys) {
+        const int dof = b->type_dof[s.type], nodes = (1 << s.bisection_level) - 1;
+        threads += (long long)s.n_walkers * (s.n_slices >> s.bisection_level);
+        if (s.bisection_level > 4) deep = true;
+        else if (nodes * (dof + (dof >= 3 ? 1 : 0)) > 30 || dof > 12) small = false;
+    }
+    const int sm_threads = small && threads > 512ll * sms * (block_threads < 512 ? 4 : 1) ? 1024 : 512;
+    // CTAs per SM, at most four (the named barriers of a CTA are a quarter of an SM's; more only to leave L1
+    // room where segments above level 4 go to the scratch buffer): a smaller CTA leaves shared memory
     // for others, unless that sends a system to device memory or has no room for a walker (24
     // clusters of 3 to 10 atoms, 256 threads, 32 a walker: one CTA per SM 1325 us a launch, two
     // 1076; 16 a walker, where two CTAs would move paths to device memory: 1551 against 2507)
-    int per_sm = std::max(1, 512 / block_threads);
+    int per_sm = std::max(1, sm_threads / block_threads);
+    if (!deep) per_sm = std::min(per_sm, 4);
     auto budget_of = [&](int k) { return k == 1 ? kTileSmem : (size_t)227 * 1024 / k - 2048; };
     for (bool fits = false; per_sm > 1 && !fits; per_sm = fits ? per_sm : per_sm / 2) {
         fits = true;
@@ -228,18 +245,36 @@ extern "C" int fs_batch_create(int32_t n_types, const int32_t *type_dof, const c
         given.push_back(s.walkers_per_tile > 0);
         s.walkers_per_tile = wpb;
     }
-    // few walkers: tiles of fewer walkers, down to a warp of threads, until every CTA has one (40
-    // walkers each of 6 small clusters, 256 threads: 18 tiles 303 us a launch, 120 tiles 132)
-    for (bool more = true; more;) {
+    // few walkers: tiles of fewer walkers, a warp of threads or more (40 walkers each of 6 small clusters, 256
+    // threads: 18 tiles 303 us a launch, 120 tiles 132).  One CTA per SM: as small as still gives every tile
+    // a CTA of its own, since a tile more waits for one (1500 of 6 atoms, N = 256, level 3, 512 threads, 152
+    // CTAs: 137 tiles 218, 188 tiles 252).  Several: halved until every CTA has a tile, past that only to four
+    // warps, for an even spread over the SMs (1500 trimers, level 3, 256 threads, 304 CTAs: 188 tiles 70, 375
+    // tiles 64; but 6000, N = 64, level 4, 64 threads, 608 CTAs: 375 tiles 121, 750 tiles 169).
+    const long long ctas = (long long)sms * std::min(4, per_sm);
+    auto tiles_of = [&](int i, int wpb) { return ((long long)b->sys[i].n_walkers + wpb - 1) / wpb; };
+    auto threads_of = [&](int i) { return b->sys[i].n_slices >> b->sys[i].bisection_level; };
+    for (int most = 32; per_sm == 1 && most < block_threads; most += 32) {
+        auto fewer = [&](int i) {
+            const int wpb = b->sys[i].walkers_per_tile;
+            return given[i] ? wpb : std::min(wpb, std::max(1, most / threads_of(i)));
+        };
+        long long tiles = 0;
+        for (int i = 0; i < n_systems; i++) tiles += tiles_of(i, fewer(i));
+        if (tiles > ctas) continue;
+        for (int i = 0; i < n_systems; i++) b->sys[i].walkers_per_tile = fewer(i);
+        break;
+    }
+    for (bool more = per_sm > 1; more;) {
         more = false;
         long long tiles = 0;
-        for (const fs_batch_system &s : b->sys) tiles += (s.n_walkers + s.walkers_per_tile - 1) / s.walkers_per_tile;
-        for (int i = 0; i < n_systems && tiles < (long long)sms * per_sm; i++) {
-            fs_batch_system &s = b->sys[i];
-            const int wpb = s.walkers_per_tile, half = (wpb + 1) / 2;
-            if (given[i] || wpb == 1 || half * (s.n_slices >> s.bisection_level) < 32) continue;
-            tiles += (s.n_walkers + half - 1) / half - (s.n_walkers + wpb - 1) / wpb;
-            s.walkers_per_tile = half;
+        for (int i = 0; i < n_systems; i++) tiles += tiles_of(i, b->sys[i].walkers_per_tile);
+        for (int i = 0; i < n_systems && tiles < ctas; i++) {
+            const int wpb = b->sys[i].walkers_per_tile, half = (wpb + 1) / 2, threads = half * threads_of(i);
+            const long long added = tiles_of(i, half) - tiles_of(i, wpb);
+            if (given[i] || wpb == 1 || threads < 32 || (threads < 128 && tiles + added > ctas)) continue;
+            tiles += added;
+            b->sys[i].walkers_per_tile = half;
             more = true;
         }
     }
@@ -287,7 +322,7 @@ extern "C" int fs_batch_create(int32_t n_types, const int32_t *type_dof, const c
     // one register budget for every CTA size up to 512, so the autotuner's candidates share
     // one compiled module
     o << "extern \"C\" __global__ void __launch_bounds__(" << (block_threads <= 512 ? 512 : block_threads)
-      << ") fs_batch_kernel(const FsBatchSys *sys, const FsBatchItem *items, int n_items, int *counter, "
+      << (sm_threads == 1024 ? ", 2" : "") << ") fs_batch_kernel(const FsBatchSys *sys, const FsBatchItem *items, int n_items, int *counter, "
          "unsigned long long old_slot)\n{\n"
          "    extern __shared__ __align__(16) float fsb_smem[];\n"
          "    __shared__ int s_it;\n"
