@@ -202,8 +202,8 @@ extern "C" int fs_batch_create(int32_t n_types, const int32_t *type_dof, const c
     // SM, for xorshift batches of at most five atoms whose segments are small (30 values: four at level 2) and whose
     // threads are many: more than a wave of 512-thread CTAs, four of smaller ones (CTAs below 256 threads
     // gain none).  Us a launch at 128 / 64, 256 and 512 threads: 6000 walkers, 3 atoms, N = 256, level 2 172 /
-    // 148 and 184 / 161; 4 atoms, N = 128, level 1 137 / 108 and 147 / 121; 5 atoms 173 / 143 and 184 / 162; 1500
-    // walkers, 3 atoms, level 2 56 / 68 and 76 / 68; level 3, 4 atoms, 6000 241 / 310 and 295 / 312.
+    // 148 and 184 / 161; 4 atoms, N = 128, level 1 137 / 108 and 146 / 121; 5 atoms 174 / 145 and 184 / 160; 1500
+    // walkers, 3 atoms, level 2 56 / 68 and 76 / 58; level 3, 4 atoms, 6000 241 / 310 and 295 / 312.
     long long threads = 0;
     bool small = b->lux < 0 && block_threads >= 256 && block_threads <= 512, deep = false;
     for (const fs_batch_system &s : b->sys) {
@@ -248,9 +248,9 @@ extern "C" int fs_batch_create(int32_t n_types, const int32_t *type_dof, const c
     // few walkers: tiles of fewer walkers, a warp of threads or more (40 walkers each of 6 small clusters, 256
     // threads: 18 tiles 303 us a launch, 120 tiles 132).  One CTA per SM: as small as still gives every tile
     // a CTA of its own, since a tile more waits for one (1500 of 6 atoms, N = 256, level 3, 512 threads, 152
-    // CTAs: 137 tiles 218, 188 tiles 252).  Several: halved until every CTA has a tile, past that only to four
+    // CTAs: 150 tiles 154, 188 tiles 252).  Several: halved until every CTA has a tile, past that only to four
     // warps, for an even spread over the SMs (1500 trimers, level 3, 256 threads, 304 CTAs: 188 tiles 70, 375
-    // tiles 64; but 6000, N = 64, level 4, 64 threads, 608 CTAs: 375 tiles 121, 750 tiles 169).
+    // tiles 64; but 6000, N = 64, level 4, 64 threads, 608 CTAs: 375 tiles 110, 750 tiles 169).
     const long long ctas = (long long)sms * std::min(4, per_sm);
     auto tiles_of = [&](int i, int wpb) { return ((long long)b->sys[i].n_walkers + wpb - 1) / wpb; };
     auto threads_of = [&](int i) { return b->sys[i].n_slices >> b->sys[i].bisection_level; };
