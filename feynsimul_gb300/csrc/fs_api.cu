@@ -133,7 +133,8 @@ struct fs_handle {
     int regs = 0;
     size_t ft = 4, op_elem = 8, cor_elem = 8;
     size_t n_ops_elems = 0, n_cor_elems = 0, n_cor_lags = 0, n_bins = 0, n_hist = 0;
-    double *d_red = nullptr;  // fs_reduce_correlator output (sum, sumsq)
+    double *d_red = nullptr;   // fs_reduce_correlator: result and partial rows, where d_cor has no room for them
+    double *d_part = nullptr;  // the same behind the correlator sums in d_cor
     void *d_shift_old = nullptr;  // path shift, fixed mode: row saved before the move
     void *d_vcache = nullptr;     // potential cache in device memory: [walkers][N]
     unsigned long long steps_done = 0;  // Metropolis steps of all launches so far
@@ -820,6 +821,17 @@ static cudaError_t drain(fs_handle *h)
     return e;
 }
 
+// Correlator moments: rows of partial sums that fs_reduce_correlator may use, two blocks per SM unless the
+// walkers are fewer or the rows would take more than 1 MB, down to one per SM, or 64 MB
+#define FS_MOM_THREADS 256
+static long long moment_rows(const fs_handle *h, size_t cols)
+{
+    const long long lags = (long long)h->cors.size() * (h->cfg.n_slices / 2), at_a_time = std::max(1ll, FS_MOM_THREADS / lags);
+    const long long bytes = (long long)(cols * sizeof(double)), small = (1ll << 20) / bytes - 1;
+    const long long room = std::max(1ll, std::min((64ll << 20) / bytes, std::max<long long>(device_sms(), small)));
+    return std::min(std::min<long long>(2ll * device_sms(), room), (h->cfg.n_walkers + at_a_time - 1) / at_a_time);
+}
+
 static int dalloc(fs_handle *h, void **p, size_t bytes)
 {
     if (bytes == 0) bytes = 16;
@@ -1142,7 +1154,13 @@ extern "C" int fs_create(const fs_config *cfg, const char *potential, const char
     h->n_bins = c.enable_bins ? (size_t)std::llround(std::pow((double)c.bin_resolution_per_dof, c.dof)) : 0;
     h->n_hist = h->hists.empty() ? 0 : (size_t)c.hist_bins;
     h->g_rows = c.compat ? T : W;
-    size_t need = W * c.dof * N * h->ft + T * 4 + h->n_ops_elems * h->op_elem + h->n_cor_lags * h->cor_elem +
+    // The moments' partial rows, up to 4 MB, behind the correlator sums: an allocation of their own in the
+    // first call took up to 100 us (340 oscillators, N = 512: a first pass with reads 277 us with it, 170 so)
+    const size_t cor_bytes = (h->n_cor_lags * h->cor_elem + 255) / 256 * 256;
+    const size_t mom_cols = 2 * h->cors.size() * (N / 2) * (c.accum == 3 ? 3 : 1);
+    const size_t mom_bytes = mom_cols ? (size_t)(moment_rows(h, mom_cols) + 1) * mom_cols * sizeof(double) : 0;
+    const size_t part_bytes = mom_bytes <= ((size_t)4 << 20) ? mom_bytes : 0;
+    size_t need = W * c.dof * N * h->ft + T * 4 + h->n_ops_elems * h->op_elem + cor_bytes + part_bytes +
                   h->n_bins * 4 + h->n_hist * 8 +
                   (c.enable_ranlux ? (T + h->g_rows) * 112 : ((T + 1) * 16 * 2 + W * 16));
     if (free_b && need > free_b) {
@@ -1167,7 +1185,8 @@ extern "C" int fs_create(const fs_config *cfg, const char *potential, const char
         CREATE_TRY(dalloc(h, (void **)&h->d_wseeds, W * 16));
     }
     CREATE_TRY(dalloc(h, &h->d_ops, h->n_ops_elems * h->op_elem));
-    CREATE_TRY(dalloc(h, &h->d_cor, h->n_cor_lags * h->cor_elem));
+    CREATE_TRY(dalloc(h, &h->d_cor, cor_bytes + part_bytes));
+    if (part_bytes) h->d_part = (double *)((char *)h->d_cor + cor_bytes);
     CREATE_TRY(dalloc(h, (void **)&h->d_bins, h->n_bins * 4));
     CREATE_TRY(dalloc(h, (void **)&h->d_hist, h->n_hist * 8));
     if ((c.moves & FS_MOVE_PATH_SHIFT) && !c.compat) CREATE_TRY(dalloc(h, &h->d_shift_old, W * N * h->ft));
@@ -1821,7 +1840,6 @@ extern "C" int fs_set_correlator(fs_handle *h, const double *in, size_t n)
 // fewer lags than threads the block takes several walkers at a time.  Stage 2 adds the rows.  No
 // atomics, so equal sums give equal bits, and nothing to clear.  Bound by its two launches:
 // 1024 walkers of 64 lags, with the read-back, 63 us before (a clear, atomics, two copies), 36 now.
-#define FS_MOM_THREADS 256
 template <int KIND>  // 0: float, 1: double, 2: study struct (3 columns)
 __global__ void __launch_bounds__(FS_MOM_THREADS) fs_cor_moments_kernel(const unsigned char *cor, int lags, long long w0,
                                                                         long long w1, double *part)
@@ -1911,17 +1929,15 @@ extern "C" int fs_reduce_correlator(fs_handle *h, int64_t walker_begin, int64_t 
         return fail(h, FS_ERR_IO, "walker range [%lld, %lld) outside [0, %zu)", (long long)walker_begin,
                     (long long)walker_end, W);
     CUDA_TRY(h, cudaSetDevice(h->device), FS_ERR_CUDA);
-    // two blocks per SM, unless the walkers are fewer or the rows would take more than 1 MB, down to
-    // one per SM (a first call that allocates more than that takes 120 us longer), or 64 MB
     const long long nw = walker_end - walker_begin, rows = std::max<long long>(1, FS_MOM_THREADS / (long long)lags);
     const size_t cols = 2 * n;
-    const long long bytes = (long long)(cols * sizeof(double)), small = (1ll << 20) / bytes - 1;
-    const long long room = std::max(1ll, std::min((64ll << 20) / bytes, std::max<long long>(device_sms(), small)));
-    const long long most = std::min(std::min<long long>(2ll * device_sms(), room), ((long long)W + rows - 1) / rows);
+    const long long most = moment_rows(h, cols);
     const unsigned grid = (unsigned)std::min(most, (nw + rows - 1) / rows);
-    if (!h->d_red) CUDA_TRY(h, cudaMalloc((void **)&h->d_red, (size_t)(most + 1) * cols * sizeof(double)), FS_ERR_OOM);
+    if (!h->d_part && !h->d_red)
+        CUDA_TRY(h, cudaMalloc((void **)&h->d_red, (size_t)(most + 1) * cols * sizeof(double)), FS_ERR_OOM);
     const unsigned char *c = (const unsigned char *)h->d_cor;
-    double *part = h->d_red + cols, *dst = h->h_red ? h->h_red : h->d_red;
+    double *const red = h->d_part ? h->d_part : h->d_red;
+    double *part = red + cols, *dst = h->h_red ? h->h_red : red;
     if (h->cor_elem == 24)
         fs_cor_moments_kernel<2><<<grid, FS_MOM_THREADS, 0, h->stream>>>(c, (int)lags, walker_begin, walker_end, part);
     else if (h->cor_elem == 8)
