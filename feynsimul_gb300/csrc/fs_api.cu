@@ -143,10 +143,10 @@ struct fs_handle {
     cudaLibrary_t lib = nullptr;
     cudaKernel_t k_metro = nullptr, k_rinit = nullptr;
     cudaStream_t stream = nullptr;
-    cudaStream_t s_in = nullptr, s_out = nullptr;  // fs_run_host copy streams
     cudaStream_t s_comp2 = nullptr;                 // fs_run_host: second compute stream
+    cudaStream_t s_in = nullptr, s_out = nullptr;   // fs_run_host, three chunks and more: copy streams
+    std::vector<cudaEvent_t> ev_chunk;              // copy-in and compute done of each chunk, and the end
     double *d_wops = nullptr;                       // fs_get_walker_operators output
-    std::vector<cudaEvent_t> ev_chunk;               // fs_run_host: copy-in / compute done per chunk
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool timed = false;
     // device buffers
@@ -1213,9 +1213,8 @@ extern "C" int fs_destroy(fs_handle *h)
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     for (cudaEvent_t e : h->ev_chunk) cudaEventDestroy(e);
-    if (h->s_in) cudaStreamDestroy(h->s_in);
-    if (h->s_out) cudaStreamDestroy(h->s_out);
-    if (h->s_comp2) cudaStreamDestroy(h->s_comp2);
+    for (cudaStream_t st : {h->s_in, h->s_comp2, h->s_out})
+        if (st) cudaStreamDestroy(st);
     if (h->lib) cudaLibraryUnload(h->lib);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
@@ -1419,11 +1418,10 @@ extern "C" int fs_run(fs_handle *h, int32_t n_launches)
 }
 
 // Pipelined run on host path buffers: the walkers are split into n_chunks CTA-aligned
-// chunks; chunk c's paths are copied in on one stream, its n_launches sweeps run on the
-// handle's stream as soon as they have arrived, and its paths are copied out on a third
-// stream while later chunks compute.  Walkers are independent, so this equals
-// set_paths + run + get_paths bit for bit (the reference-compatible xorshift mode, whose
-// walker streams read other walkers' seed rows, runs as one chunk).
+// chunks, whose n_launches sweeps alternate between two streams: a chunk's paths are copied in
+// while the chunk before computes and copied out while the one behind it does.  Walkers are
+// independent, so this equals set_paths + run + get_paths bit for bit (the reference-compatible
+// xorshift mode, whose walker streams read other walkers' seed rows, runs as one chunk).
 extern "C" int fs_run_host(fs_handle *h, const void *paths_in, void *paths_out, int32_t n_launches,
                            int32_t n_chunks)
 {
@@ -1479,64 +1477,91 @@ extern "C" int fs_run_host(fs_handle *h, const void *paths_in, void *paths_out, 
         h->status_pending = true;
         return FS_OK;
     }
-    if (!h->s_in) CUDA_TRY(h, cudaStreamCreateWithFlags(&h->s_in, cudaStreamNonBlocking), FS_ERR_CUDA);
-    if (!h->s_out) CUDA_TRY(h, cudaStreamCreateWithFlags(&h->s_out, cudaStreamNonBlocking), FS_ERR_CUDA);
-    if (!h->s_comp2) CUDA_TRY(h, cudaStreamCreateWithFlags(&h->s_comp2, cudaStreamNonBlocking), FS_ERR_CUDA);
-    while ((int)h->ev_chunk.size() < 2 * n_chunks + 2) {
-        cudaEvent_t e;
-        CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), FS_ERR_CUDA);
-        h->ev_chunk.push_back(e);
-    }
-    CUDA_TRY(h, cudaEventRecord(h->ev0, h->stream), FS_ERR_CUDA);
-    // the copy streams start after everything queued before this call
-    CUDA_TRY(h, cudaStreamWaitEvent(h->s_in, h->ev0, 0), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamWaitEvent(h->s_out, h->ev0, 0), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamWaitEvent(h->s_comp2, h->ev0, 0), FS_ERR_CUDA);
     // chunks alternate between two compute streams, so one chunk's last wave overlaps the
     // next chunk's first (they touch disjoint walkers; shared histograms use atomics).  With
     // three or more chunks the first and the last are a third of the others: only the first
     // chunk's copy in and the last chunk's copy out are not hidden behind sweeps.
-    cudaStream_t comp[2] = {h->stream, h->s_comp2};
     const long long wsum = n_chunks >= 3 ? 3ll * (n_chunks - 2) + 2 : n_chunks;
     auto cut = [&](int k) -> int {  // first CTA of chunk k (k = n_chunks: the grid)
         long long wk = n_chunks >= 3 ? (k == 0 ? 0 : 1 + 3ll * (std::min(k, n_chunks - 1) - 1) + (k == n_chunks ? 1 : 0))
                                      : k;
         return (int)((long long)h->grid * wk / wsum);
     };
-    for (int k = 0; k < n_chunks; k++) {
-        const int cta0 = cut(k);
-        const int cta1 = cut(k + 1);
-        const size_t w0 = (size_t)cta0 * h->wpb;
-        const size_t w1 = std::min((size_t)cta1 * h->wpb, (size_t)c.n_walkers);
-        if (cta1 <= cta0 || w1 <= w0) continue;
-        cudaEvent_t e_in = h->ev_chunk[2 * k], e_done = h->ev_chunk[2 * k + 1];
-        CUDA_TRY(h, cudaMemcpyAsync((char *)h->d_paths + w0 * bpw, (const char *)paths_in + w0 * bpw, (w1 - w0) * bpw,
-                                    cudaMemcpyHostToDevice, h->s_in), FS_ERR_CUDA);
-        CUDA_TRY(h, cudaEventRecord(e_in, h->s_in), FS_ERR_CUDA);
-        cudaStream_t cs = comp[k & 1];
-        CUDA_TRY(h, cudaStreamWaitEvent(cs, e_in, 0), FS_ERR_CUDA);
-        a.block_offset = cta0;
-        for (int i = 0; i < n_launches; i++) {
+    struct Part { int cta0, ctas; size_t from, bytes; };
+    auto part = [&](int k) {
+        const int cta0 = cut(k), cta1 = cut(k + 1);
+        const size_t w0 = (size_t)cta0 * h->wpb, w1 = std::min((size_t)cta1 * h->wpb, (size_t)c.n_walkers);
+        return cta1 <= cta0 || w1 <= w0 ? Part{cta0, 0, 0, 0} : Part{cta0, cta1 - cta0, w0 * bpw, (w1 - w0) * bpw};
+    };
+    auto copy_in = [&](const Part &p, cudaStream_t st) {
+        return cudaMemcpyAsync((char *)h->d_paths + p.from, (const char *)paths_in + p.from, p.bytes,
+                               cudaMemcpyHostToDevice, st);
+    };
+    auto sweeps = [&](const Part &p, cudaStream_t st) {
+        a.block_offset = p.cta0;
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; e == cudaSuccess && i < n_launches; i++) {
             a.step_base = h->steps_done + per_launch * (unsigned long long)i;
-            if (h->d_snap)
-                CUDA_TRY(h, cudaMemcpyAsync(h->d_snap, h->d_seeds, (h->n_threads + 1) * 16, cudaMemcpyDeviceToDevice,
-                                            cs), FS_ERR_CUDA);
-            CUDA_TRY(h, cudaLaunchKernel((const void *)h->k_metro, dim3(cta1 - cta0), dim3(h->block), args, h->smem,
-                                         cs), FS_ERR_LAUNCH);
+            e = cudaLaunchKernel((const void *)h->k_metro, dim3(p.ctas), dim3(h->block), args, h->smem, st);
         }
-        CUDA_TRY(h, cudaEventRecord(e_done, cs), FS_ERR_CUDA);
-        CUDA_TRY(h, cudaStreamWaitEvent(h->s_out, e_done, 0), FS_ERR_CUDA);
-        CUDA_TRY(h, cudaMemcpyAsync((char *)paths_out + w0 * bpw, (const char *)h->d_paths + w0 * bpw, (w1 - w0) * bpw,
-                                    cudaMemcpyDeviceToHost, h->s_out), FS_ERR_CUDA);
+        return e;
+    };
+    // Two chunks keep to a compute stream each, copies too; more have copy streams.  In a first call, the first
+    // chunk goes in order on the handle's stream and the other streams and events are made behind it: they
+    // take 30 us a stream (first passes of trimers, N = 128, with reads, one chunk / two on four streams made
+    // first / two so: 1000 walkers 403 / 425 / 330, 2500 545 / 565 / 437, xorshift 2500 382 / 475 / 425).
+    // ev1 is the end of the first chunk's copy here.
+    const Part first = part(0);
+    const bool own = n_chunks > 2;
+    cudaStream_t in0 = own && h->s_in ? h->s_in : h->stream;
+    CUDA_TRY(h, cudaEventRecord(h->ev0, h->stream), FS_ERR_CUDA);
+    if (in0 != h->stream) CUDA_TRY(h, cudaStreamWaitEvent(in0, h->ev0, 0), FS_ERR_CUDA);
+    if (first.ctas) CUDA_TRY(h, copy_in(first, in0), FS_ERR_CUDA);
+    CUDA_TRY(h, cudaEventRecord(h->ev1, in0), FS_ERR_CUDA);
+    if (in0 != h->stream) CUDA_TRY(h, cudaStreamWaitEvent(h->stream, h->ev1, 0), FS_ERR_CUDA);
+    if (first.ctas) CUDA_TRY(h, sweeps(first, h->stream), FS_ERR_LAUNCH);
+    for (cudaStream_t *st : {&h->s_comp2, &h->s_in, &h->s_out})
+        if (!*st && (own || st == &h->s_comp2))
+            CUDA_TRY(h, cudaStreamCreateWithFlags(st, cudaStreamNonBlocking), FS_ERR_CUDA);
+    while ((int)h->ev_chunk.size() < (own ? 2 * n_chunks + 1 : 1)) {
+        cudaEvent_t e;
+        CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), FS_ERR_CUDA);
+        h->ev_chunk.push_back(e);
+    }
+    cudaStream_t comp[2] = {h->stream, h->s_comp2};
+    // the other streams start after everything queued before this call, and the copies in go one by one
+    CUDA_TRY(h, cudaStreamWaitEvent(h->s_comp2, h->ev1, 0), FS_ERR_CUDA);
+    if (own) {
+        if (in0 != h->s_in) CUDA_TRY(h, cudaStreamWaitEvent(h->s_in, h->ev1, 0), FS_ERR_CUDA);
+        CUDA_TRY(h, cudaStreamWaitEvent(h->s_out, h->ev0, 0), FS_ERR_CUDA);
+    }
+    for (int k = 0; k < n_chunks; k++) {
+        const Part p = part(k);
+        if (!p.ctas) continue;
+        cudaStream_t cs = comp[k & 1], in = own ? h->s_in : cs, out = own ? h->s_out : cs;
+        if (k > 0) {
+            CUDA_TRY(h, copy_in(p, in), FS_ERR_CUDA);
+            if (own) {
+                CUDA_TRY(h, cudaEventRecord(h->ev_chunk[2 * k], in), FS_ERR_CUDA);
+                CUDA_TRY(h, cudaStreamWaitEvent(cs, h->ev_chunk[2 * k], 0), FS_ERR_CUDA);
+            }
+            CUDA_TRY(h, sweeps(p, cs), FS_ERR_LAUNCH);
+        }
+        if (own) {
+            CUDA_TRY(h, cudaEventRecord(h->ev_chunk[2 * k + 1], cs), FS_ERR_CUDA);
+            CUDA_TRY(h, cudaStreamWaitEvent(out, h->ev_chunk[2 * k + 1], 0), FS_ERR_CUDA);
+        }
+        CUDA_TRY(h, cudaMemcpyAsync((char *)paths_out + p.from, (const char *)h->d_paths + p.from, p.bytes,
+                                    cudaMemcpyDeviceToHost, out), FS_ERR_CUDA);
     }
     h->steps_done += per_launch * (unsigned long long)n_launches;
-    // the handle's stream (fs_sync, the getters) waits for the second compute stream and
-    // the last copy out
-    cudaEvent_t e_end = h->ev_chunk[2 * n_chunks], e_c2 = h->ev_chunk[2 * n_chunks + 1];
-    CUDA_TRY(h, cudaEventRecord(e_end, h->s_out), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaEventRecord(e_c2, h->s_comp2), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamWaitEvent(h->stream, e_end, 0), FS_ERR_CUDA);
-    CUDA_TRY(h, cudaStreamWaitEvent(h->stream, e_c2, 0), FS_ERR_CUDA);
+    // the handle's stream (fs_sync, the getters) waits for the second compute stream and the last copy out
+    CUDA_TRY(h, cudaEventRecord(h->ev_chunk[0], h->s_comp2), FS_ERR_CUDA);
+    CUDA_TRY(h, cudaStreamWaitEvent(h->stream, h->ev_chunk[0], 0), FS_ERR_CUDA);
+    if (own) {
+        CUDA_TRY(h, cudaEventRecord(h->ev_chunk[2 * n_chunks], h->s_out), FS_ERR_CUDA);
+        CUDA_TRY(h, cudaStreamWaitEvent(h->stream, h->ev_chunk[2 * n_chunks], 0), FS_ERR_CUDA);
+    }
     CUDA_TRY(h, cudaEventRecord(h->ev1, h->stream), FS_ERR_CUDA);
     h->timed = true;
     h->status_pending = true;

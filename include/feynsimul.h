@@ -203,7 +203,7 @@ int fs_set_ranlux_tables(fs_handle *h, const uint32_t *tab, size_t n_tab_rows,
 int fs_run(fs_handle *h, int32_t n_launches);
 /* n_launches runs on host path buffers ([walkers][DOF][N] in the path precision; in and
  * out may be the same buffer), pipelined: the walkers are split into n_chunks chunks whose
- * copy-in, sweeps and copy-out overlap on three streams (n_chunks = 0: automatic, up to 6
+ * copy-in, sweeps and copy-out overlap on two to four streams (n_chunks = 0: automatic, up to 6
  * chunks; one where the CTAs are less than a quarter of a wave).  Equivalent to fs_set_paths +
  * fs_run + fs_get_paths (kernel.py:567-574, :459-506, :557-565); asynchronous like fs_run
  * (the buffers must stay valid until fs_sync), and overlapping only for page-locked host
