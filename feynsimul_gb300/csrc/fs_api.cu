@@ -1029,11 +1029,26 @@ static int prepare(const fs_config *cfg, const char *potential, const char *user
             (long long)c.operator_runs * c.metro_steps_per_operator_run >= 2)
             h->vglobal = 1;
     }
-    if (h->smem > room) {
-        // the bank spread is not worth a CTA that fits without it
-        if (!c.global_path) h->wstride = round16((long long)c.dof * dstride);
-        if (h->vstride) h->vstride = round16(dstride);
-        h->smem = sweep_smem(*h, h->vstride, hist_bytes);
+    // The bank spread is not worth a CTA: neither the only one that fits, nor one more on an SM (228 KB, 1
+    // of them the system's for each CTA) where the grid has one to put there.  Then strides of an odd multiple
+    // of 16 words, with which two walkers of a warp use opposite bank halves, or of 16 words (8000 of 5 atoms,
+    // N = 64, S = 4: 57856 bytes, three CTAs per SM, 504 us a run; 57344, four, 319).
+    auto resident = [&](size_t smem) {
+        return std::min(std::min((228ll * 1024) / (long long)(smem + 1024), 2048ll / h->block),
+                        (long long)(h->grid + device_sms() - 1) / device_sms());
+    };
+    for (int odd = 1; odd >= 0; odd--) {
+        auto stride = [&](long long words) { return round16(words) + (odd && round16(words) / 16 % 2 == 0 ? 16 : 0); };
+        const long long w = h->wstride, v = h->vstride;
+        if (!c.global_path) h->wstride = stride((long long)c.dof * dstride);
+        if (h->vstride) h->vstride = stride(dstride);
+        const size_t smem = sweep_smem(*h, h->vstride, hist_bytes);
+        if (smem < h->smem && (h->smem > room || resident(smem) > resident(h->smem))) {
+            h->smem = smem;
+        } else {
+            h->wstride = w;
+            h->vstride = v;
+        }
     }
     // Register budget: unless the caller fixes it, compile for as many CTAs per SM as shared
     // memory admits (<= 2048 threads per SM, >= 64 registers per thread) and as the grid can
