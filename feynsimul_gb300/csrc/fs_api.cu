@@ -669,8 +669,10 @@ static int default_wpb(const fs_handle &h, size_t per_walker, size_t hist_bytes)
 // 388 / - / -; trimer RANLUX (50) 136 / 116 / 103 / 101, (150) 136 / 116 / 104 / 125, (300) 121 / 105 / 106
 // / 149, (600) 141 / 146 / 207 / 360; 10 atoms (150) 398 / 188 / 127 / 125, (1000) 202 / 286 / 247 / 247;
 // 5 atoms FP64 (50) 4676 / 2855 / 1619 / 1194, (200) 4678 / 3225 / 2324 / 2638, (512) 5170 / 5520 / 4551 /
-// 5653.  With segments of 4 slices a trimer's lanes have too little to share (T = 64: 51 / 56 / 67,
-// FP64 749 / 480 / 545).  Twelve-value RANLUX draws need at most 8 degrees of freedom here, and
+// 5653; trimers FP64 RANLUX, S = 3 (375) 2180 / 2279 / 1876, (464) 2185 / 2286 / 2454, 4 atoms (464) 3955 / 4329 /
+// 4438.  With segments of 8 slices and fewer the lanes share less (trimer, fast: S = 3 (250) 38 / 32 / 32,
+// (375) 38.3 / 40.6; S = 2 (250) 19.8 / 18.5, (500) 19.9 / 22.7), and with 4 slices a trimer's too little across
+// warps (T = 64: 51 / 56 / 67, FP64 749 / 480 / 545).  Twelve-value RANLUX draws need at most 8 degrees of freedom here, and
 // potentials of one or two degrees have nothing to share.
 static int lanes_for(const fs_handle &h)
 {
@@ -684,8 +686,8 @@ static int lanes_for(const fs_handle &h)
         int lanes;
         double most;  // warps per scheduler with them
     } rule[] = {{8, dbl || !c.fast_math ? 1.5 : 0.66},
-                {4, dbl ? 3.4 : !c.fast_math ? 2.0 : 1.0},
-                {2, dbl ? 1.0 : ranlux ? 1.6 : 2.0}};
+                {4, dbl ? (c.dof >= 12 ? 3.4 : 2.5) : !c.fast_math ? 2.0 : 1.0},
+                {2, dbl ? 1.0 : c.fast_math && h.seg < 16 ? 1.0 : ranlux ? 1.6 : 2.0}};
     for (const auto &r : rule) {
         if (r.lanes > h.seg || r.lanes * h.tpw > 1024 || warps * r.lanes > r.most * schedulers) continue;
         if (c.min_blocks_per_sm * r.lanes * h.tpw > 2048) continue;  // the caller's CTAs per SM
