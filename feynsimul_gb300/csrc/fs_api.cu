@@ -362,6 +362,8 @@ struct GenOut {
     std::string src;
 };
 
+static int device_sms();
+
 static std::string gen_source(const fs_handle &h, const std::string &potential,
                               const std::string &user_code)
 {
@@ -393,7 +395,7 @@ static std::string gen_source(const fs_handle &h, const std::string &potential,
       << "\n#define FS_VCACHE " << (h.vstride || h.vglobal ? 1 : 0) << "\n#define FS_VSTRIDE " << h.vstride
       << "\n#define FS_VGLOBAL " << h.vglobal
       << "\n#define FS_COR_ILV " << h.cor_ilv << "\n#define FS_CWSTRIDE " << h.cwstride << "\n#define FS_MX "
-      << h.mx << "\n#define FS_PIPE " << h.pipe << "\n#define FS_PLAGS " << h.plags << "\n#define FS_CONSEC " << h.consec << "\n#define FS_SNSTRIDE " << h.snstride << "\n#define FS_G " << h.lanes << "\n";
+      << h.mx << "\n#define FS_PIPE " << h.pipe << "\n#define FS_PLAGS " << h.plags << "\n#define FS_CONSEC " << h.consec << "\n#define FS_SNSTRIDE " << h.snstride << "\n#define FS_G " << h.lanes << "\n#define FS_SMS " << device_sms() << "\n";
     {
         const int mv = c.moves ? c.moves : FS_MOVE_BISECTION;
         const double nb = (double)c.n_slices / c.beta;

@@ -280,14 +280,22 @@ __device__ __forceinline__ fs_u32 fs_offset(FsIStream &g, fs_u32 range)
 // line lies at 3000.  Rolled, a fast trimer gains 1 % from two nodes at a time, an IEEE one loses
 // 9 % (its six degrees fill the cache), and a cheap potential wants its action loop unrolled
 // (oscillator IEEE S = 6: 1053 against 1326).
+// One exception: with pipelined correlator helpers, of whose CTAs an SM then holds one warp of movers each, and
+// more than three such CTAs per SM, a trimer's fast S = 4 move of 4 or 8 threads a walker is the faster one
+// unrolled (us a run, unrolled / rolled: N = 64, 1000 walkers 90 / 72, 5000 114 / 145, 8000 209 / 252, 16000 358 /
+// 390; N = 128, 1000 90 / 73, 2500 113 / 143, 5000 240 / 261, 8000 370 / 385).  Not at S = 3 (N = 64, 8000 163 /
+// 145), nor with 2 or 16 threads (N = 32, 8000 110 / 90; N = 256, 16000 1564 / 1417).
 // RANLUX (its generator calls are large) and more than 8 degrees of freedom are always rolled.
+#define FS_MOVE_FULL                                                                                              \
+    (FS_MOVE_CODE <= 3000 || (FS_PIPE && FS_DOF > 2 && FS_MOVE_CODE > 5000 && FS_MOVE_CODE <= 8000 && FS_TPW >= 4 && \
+                              FS_TPW <= 8 && FS_NWALKERS > 3 * FS_SMS * FS_WPB))
 #define FS_MOVE_CODE ((FS_SEG - 1) * (FS_DOF * (FS_FAST ? 30 : 180) + (FS_DOF < 3 ? 10 : 50 * FS_DOF)))
 #if FS_RANLUX || FS_DOF > 8
 #define FS_MOVE_UNROLL _Pragma("unroll 1")
 #define FS_NODE_UNROLL _Pragma("unroll 1")
 #define FS_DOF_UNROLL _Pragma("unroll 1")
 #define FS_ACT_UNROLL _Pragma("unroll 1")
-#elif FS_MOVE_CODE <= 3000
+#elif FS_MOVE_FULL
 #define FS_MOVE_UNROLL _Pragma("unroll")
 #define FS_NODE_UNROLL _Pragma("unroll")
 #define FS_DOF_UNROLL _Pragma("unroll")
